@@ -78,6 +78,10 @@ inline int64_t grid_cap_nr(const sopb_params& p, int64_t cap_pp, int64_t cap_pl)
     return near_skin(p) > 0.02f ? std::max<int64_t>(1, std::min<int64_t>(cap_pp, 2 * cap_pl)) : 0;
 }
 
+// Entries of a resident job's row of two beads with at most cap_pl partners
+// each: the Verlet rows (mult 2), the near rows (mult 4).
+inline int64_t row_cap(int64_t n, int64_t cap_pl, int mult) { return std::max<int64_t>(1, std::min<int64_t>(n, mult * cap_pl)); }
+
 // Default CTAs per SM that the O(N^2) TEA and D F sums are sliced for (the
 // fastest of 2..32 for TEA and exact HI at 4000 beads on B200).
 constexpr int32_t kHiCtasPerSm = 8;
@@ -95,6 +99,9 @@ struct ShapePolicy {
 
 struct LaunchClass {
     int block = 0;
+    int cluster = 1;              // CTAs per job
+    int lpb = 0;                  // lanes per bead
+    bool wide = false;            // a lane group of twice the usual width per pair of beads
     int32_t max_n = 0;
     size_t smem = 0;
     std::vector<int32_t> ids;
@@ -168,7 +175,8 @@ struct sopb_context {
     int smem_dyn_max = 1 << 30;   // dynamic shared memory available to the resident kernel
     int smem_per_sm = 0;          // shared memory of one SM
     int smem_reserved = 0;        // shared memory the runtime reserves per CTA
-    int smem_static[5] = {};      // static shared memory of k_resident_steps<64..1024>
+    int smem_static = 0;          // static shared memory of k_resident_steps
+    int cluster_ctas[kClusterSizes] = {};   // CTAs of clusters of 1, 2, 4, .. that run at once, one per SM
     ShapePolicy policy;
 };
 
@@ -240,23 +248,22 @@ void hi_streams_destroy(sopb_job* j) {
     for (cudaEvent_t e : j->lk_ev) if (e) cudaEventDestroy(e);
 }
 
-// Opt the resident kernel in to the largest dynamic shared memory the device
+// Opt a resident kernel in to the largest dynamic shared memory the device
 // allows next to the kernel's static shared memory.
-template <int B>
+template <bool CL, bool WIDE, int G>
 int set_smem_attr(int device, int* dyn_out, int* static_out) {
     int optin = 0;
     CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
     cudaFuncAttributes fa;
-    CUDA_TRY(cudaFuncGetAttributes(&fa, k_resident_steps<B>));
+    CUDA_TRY(cudaFuncGetAttributes(&fa, k_resident_steps<CL, WIDE, G>));
     const int dyn = optin - (int)fa.sharedSizeBytes;
     if (dyn < kMaxResidentBeads * kResidentSmemPerBead) return SOPB_ERR_UNSUPPORTED;
-    CUDA_TRY(cudaFuncSetAttribute(k_resident_steps<B>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
+    CUDA_TRY(cudaFuncSetAttribute(k_resident_steps<CL, WIDE, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
+    if (CL) CUDA_TRY(cudaFuncSetAttribute(k_resident_steps<CL, WIDE, G>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     if (dyn < *dyn_out) *dyn_out = dyn;
-    *static_out = (int)fa.sharedSizeBytes;
+    *static_out = std::max(*static_out, (int)fa.sharedSizeBytes);
     return SOPB_OK;
 }
-
-int block_index(int block) { return block == 64 ? 0 : block == 128 ? 1 : block == 256 ? 2 : block == 512 ? 3 : 4; }
 
 // Smallest float t with sqrtf(t) >= cut: for every float r2,
 // sqrtf(r2) < cut exactly when r2 < t, because a correctly rounded square
@@ -293,37 +300,45 @@ void launch_shape(const ShapePolicy& pol, int32_t n, int32_t lpb_req, int32_t* l
     *block = b;
 }
 
-#define SOPB_BLOCK_SWITCH(block, LAUNCH) \
-    switch (block) {                      \
-    case 64: LAUNCH(64); break;           \
-    case 128: LAUNCH(128); break;         \
-    case 256: LAUNCH(256); break;         \
-    case 512: LAUNCH(512); break;         \
-    case 1024: LAUNCH(1024); break;       \
-    default: return SOPB_ERR_INVALID;     \
-    }
+// A resident launch of `njobs` jobs with `cluster` CTAs each.
+cudaLaunchConfig_t resident_config(int block, int cluster, int njobs, size_t smem, cudaStream_t st, cudaLaunchAttribute* at) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(njobs * cluster));
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    at->id = cudaLaunchAttributeClusterDimension;
+    at->val.clusterDim = {(unsigned)cluster, 1, 1};
+    cfg.attrs = at;
+    cfg.numAttrs = cluster > 1 ? 1 : 0;
+    return cfg;
+}
 
-int launch_resident(int block, int grid, size_t smem, cudaStream_t st, JobDev* jobs, const int32_t* ids,
-                    const int64_t* steps) {
-#define L_RES(B) k_resident_steps<B><<<grid, B, smem, st>>>(jobs, ids, steps)
-    SOPB_BLOCK_SWITCH(block, L_RES)
-#undef L_RES
+// The kernel of a class: one CTA per job or a cluster; the usual four lanes
+// per bead or any other number.
+using ResidentKernel = void (*)(JobDev*, const int32_t*, const int64_t*);
+ResidentKernel resident_kernel(const LaunchClass& L) {
+    if (L.wide) return k_resident_steps<true, true, 16>;
+    if (L.cluster > 1) return L.lpb == 4 ? k_resident_steps<true, false, 8> : k_resident_steps<true, false, 0>;
+    return L.lpb == 4 ? k_resident_steps<false, false, 8> : k_resident_steps<false, false, 0>;
+}
+
+int launch_resident(const LaunchClass& L, cudaStream_t st, JobDev* jobs, const int32_t* ids, const int64_t* steps) {
+    cudaLaunchAttribute at;
+    const cudaLaunchConfig_t cfg = resident_config(L.block, L.cluster, (int)L.ids.size(), L.smem, st, &at);
+    CUDA_TRY(cudaLaunchKernelEx(&cfg, resident_kernel(L), jobs, ids, steps));
     CUDA_TRY(cudaGetLastError());
     return SOPB_OK;
 }
 
 int launch_forces(int block, int grid, cudaStream_t st, const JobDev* jobs, const int32_t* ids, float4* out) {
-#define L_FRC(B) k_forces_only<B><<<grid, B, 0, st>>>(jobs, ids, out)
-    SOPB_BLOCK_SWITCH(block, L_FRC)
-#undef L_FRC
+    k_forces_only<<<grid, block, 0, st>>>(jobs, ids, out);
     CUDA_TRY(cudaGetLastError());
     return SOPB_OK;
 }
 
 int launch_rebuild(int block, int grid, cudaStream_t st, JobDev* jobs, const int32_t* ids, int possible, int verlet) {
-#define L_REB(B) k_rebuild_lists<B><<<grid, B, 0, st>>>(jobs, ids, possible, verlet)
-    SOPB_BLOCK_SWITCH(block, L_REB)
-#undef L_REB
+    k_rebuild_lists<<<grid, block, 0, st>>>(jobs, ids, possible, verlet);
     CUDA_TRY(cudaGetLastError());
     return SOPB_OK;
 }
@@ -483,12 +498,24 @@ extern "C" int sopb_context_create(int32_t device, void* stream, sopb_context** 
     CUDA_TRY(cudaStreamCreateWithFlags(&c->upload, cudaStreamNonBlocking));
     CUDA_TRY(cudaStreamCreateWithFlags(&c->io, cudaStreamNonBlocking));
     int rc;
-    int* dm = &c->smem_dyn_max;
-    int* ss = c->smem_static;
-    if ((rc = set_smem_attr<64>(device, dm, &ss[0])) || (rc = set_smem_attr<128>(device, dm, &ss[1])) ||
-        (rc = set_smem_attr<256>(device, dm, &ss[2])) || (rc = set_smem_attr<512>(device, dm, &ss[3])) ||
-        (rc = set_smem_attr<1024>(device, dm, &ss[4])))
+    int *dm = &c->smem_dyn_max, *ss = &c->smem_static;
+    if ((rc = set_smem_attr<false, false, 8>(device, dm, ss)) || (rc = set_smem_attr<false, false, 0>(device, dm, ss)) ||
+        (rc = set_smem_attr<true, false, 8>(device, dm, ss)) || (rc = set_smem_attr<true, false, 0>(device, dm, ss)) ||
+        (rc = set_smem_attr<true, true, 16>(device, dm, ss)))
         return rc;
+    // CTAs that clusters of each size can occupy at once with one CTA per SM
+    // (a cluster lies within one GPC, so the larger ones reach fewer SMs)
+    c->cluster_ctas[0] = c->sm_count;
+    for (int k = 1; k < kClusterSizes; ++k) {
+        cudaLaunchAttribute at;
+        const cudaLaunchConfig_t cfg = resident_config(kClusterBlock, 1 << k, 1, (size_t)c->smem_dyn_max, nullptr, &at);
+        int clusters = 0;
+        if (cudaOccupancyMaxActiveClusters(&clusters, k_resident_steps<true, false, 8>, &cfg) != cudaSuccess) {
+            cudaGetLastError();   // this size does not run here
+            clusters = 0;
+        }
+        c->cluster_ctas[k] = clusters << k;
+    }
     CUDA_TRY(cudaDeviceGetAttribute(&c->smem_per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, device));
     CUDA_TRY(cudaFuncSetAttribute(k_chol_potrf64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPotrfSmem));
     CUDA_TRY(cudaFuncSetAttribute(k_chol_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem));
@@ -1127,6 +1154,68 @@ int grid_run(sopb_job* j, cudaStream_t st, int64_t nsteps) {
 
 }  // namespace
 
+namespace {
+// in[q] = 1 where bead q is closer to bead i than the root of cut2 (x: the
+// coordinates, one component after another).
+__attribute__((optimize("O3"))) void within(const float* x, int32_t n, int32_t i, float cut2, uint8_t* in) {
+    const float *y = x + n, *z = y + n, xi = x[i], yi = y[i], zi = z[i];
+    for (int32_t q = 0; q < n; ++q) {
+        const float dx = x[q] - xi, dy = y[q] - yi, dz = z[q] - zi;
+        in[q] = dx * dx + dy * dy + dz * dz < cut2;
+    }
+}
+
+// Shared-memory needs of a resident job's CTAs for each cluster size: the
+// bonded map entries of a CTA's beads, whether the maps fit beside the
+// per-bead state, and the room for its Verlet rows -- the rows at the initial
+// coordinates plus 10 % and 4 entries per bead, as far as it fits.
+void resident_shapes(const sopb_context* c, const sopb_job_desc* d, const HostMaps& m, float cut, JobDev& h) {
+    const int32_t n = d->n, np = job_pairs(n);
+    std::vector<float> x(3 * (size_t)n);
+    for (int32_t i = 0; i < n; ++i)
+        for (int c2 = 0; c2 < 3; ++c2) x[(size_t)c2 * n + i] = d->xyz[3 * i + c2];
+    std::vector<uint8_t> in(2 * (size_t)n);
+    std::vector<int64_t> upto(np + 1, 0);                 // row entries of the pairs before
+    for (int32_t p = 0; p < np; ++p) {
+        for (int32_t h2 = 0; h2 < 2; ++h2) {
+            const int32_t i = 2 * p + h2;
+            uint8_t* row = in.data() + (size_t)h2 * n;
+            if (i >= n) {
+                std::fill(row, row + n, uint8_t(0));
+                continue;
+            }
+            within(x.data(), n, i, cut * cut, row);
+            row[i] = 0;
+            for (int32_t k = m.cov_off[i]; k < m.cov_off[i + 1]; ++k) row[m.cov_j[k]] = 0;
+            for (int32_t k = m.nat_off[i]; k < m.nat_off[i + 1]; ++k) row[m.nat_j[k]] = 0;
+        }
+        int64_t len = 0;
+        for (int32_t q = 0; q < n; ++q) len += in[q] | in[(size_t)n + q];
+        upto[p + 1] = upto[p] + len;
+    }
+    for (int k = 0; k < kClusterSizes; ++k) {
+        const int C = 1 << k;
+        int32_t ncov = 0, nnat = 0;
+        int64_t rows = 0;
+        for (int r = 0; r < C; ++r) {
+            const int p0 = pair_begin(n, r, C), p1 = pair_begin(n, r + 1, C);
+            const int32_t b0 = std::min(n, 2 * p0), b1 = std::min(n, 2 * p1);
+            ncov = std::max(ncov, m.cov_off[b1] - m.cov_off[b0]);
+            nnat = std::max(nnat, m.nat_off[b1] - m.nat_off[b0]);
+            rows = std::max(rows, upto[p1] - upto[p0]);
+        }
+        h.lcov[k] = ncov;
+        h.lnat[k] = nnat;
+        const size_t dyn = (size_t)c->smem_dyn_max;
+        // 16-bit offsets into a CTA's maps
+        h.bsm[k] = ncov < 65536 && nnat < 65536 && resident_layout(n, C, ncov, nnat, 1, 0).total <= dyn ? 1 : 0;
+        const int64_t want = (int64_t)std::ceil(1.10 * (double)rows) + 4 * (int64_t)local_beads_max(n, C);
+        const int64_t fit = ((int64_t)dyn - (int64_t)resident_layout(n, C, ncov, nnat, h.bsm[k], 0).total - 16) / 2;
+        h.lcache[k] = (int32_t)std::max<int64_t>(0, std::min(want, fit));
+    }
+}
+}  // namespace
+
 extern "C" int sopb_job_footprint(const sopb_job_desc* d, size_t* bytes) {
     if (!d || !bytes || d->n <= 0) return SOPB_ERR_INVALID;
     const int64_t n = d->n;
@@ -1138,17 +1227,19 @@ extern "C" int sopb_job_footprint(const sopb_job_desc* d, size_t* bytes) {
     b += align256((n + 1) * 4) * 2;                 // offsets
     b += align256(2 * (size_t)d->nbonds * 8);       // cov_j + r0
     b += align256(2 * (size_t)d->nnatives * 12);    // nat_j + par
-    b += align256(n * 4) * 2;                       // counts
     if (grid) {
+        b += align256(n * 4) * 2;                   // counts
         b += align256(n * cap_pp * 4);              // possible-pair rows
     } else {
         const int64_t W = (n + 31) / 32;
         b += 2 * align256(n * W * 4);               // exclusion and possible-pair masks
-        // near list (u16 rows) and the coordinates it was built at
-        b += align256(n * std::max<int64_t>(1, std::min<int64_t>(n - 1, 2 * cap_pl)) * 2) + align256(n * 4) +
-             align256(n * 16);
+        // Verlet rows and near rows of the pairs of beads (u16), their headers
+        // and the coordinates the near rows were built at
+        const int64_t np = job_pairs((int)n);
+        b += align256(np * 8) + align256(np * row_cap(n, cap_pl, 2) * 2);
+        b += align256(np * row_cap(n, cap_pl, 4) * 2) + align256(np * 4) + align256(n * 16);
     }
-    b += align256(n * cap_pl * 4);                  // Verlet rows
+    if (grid) b += align256(n * cap_pl * 4);        // Verlet rows
     b += n * (16 + 16 + 16 + 4 + 16 + 1);           // bead pools
     if ((p.pulling && p.deltax != 0.0f) || p.indentation || p.pullingPlane)
         b += align256((size_t)(p.log_rows > 0 ? p.log_rows : 1024) * 64);                        // event log
@@ -1371,32 +1462,7 @@ extern "C" int sopb_job_create(sopb_context* c, const sopb_job_desc* d, sopb_job
     }
     h.W = (n + 31) / 32;
     h.mask = h.grid ? 0 : 1;
-    h.ncov = m.cov_off[n];
-    h.nnat = m.nat_off[n];
-    if (!h.grid) {
-        // bonded maps in shared memory when they fit beside the per-bead
-        // state; then a cache of the Verlet list: the list at the initial
-        // coordinates plus 10% and 4 entries per bead, as far as it fits
-        h.bsm = resident_layout(n, h.ncov, h.nnat, 1, 0).total <= (size_t)c->smem_dyn_max ? 1 : 0;
-        const float cut = std::min(p.pairlist_cutoff, p.pairs_threshold);
-        std::vector<uint8_t> bonded((size_t)n * n, 0);
-        for (int32_t i = 0; i < n; ++i) {
-            for (int32_t k = m.cov_off[i]; k < m.cov_off[i + 1]; ++k) bonded[(size_t)i * n + m.cov_j[k]] = 1;
-            for (int32_t k = m.nat_off[i]; k < m.nat_off[i + 1]; ++k) bonded[(size_t)i * n + m.nat_j[k]] = 1;
-        }
-        int64_t total = 0;
-        for (int32_t i = 0; i < n; ++i)
-            for (int32_t q = i + 1; q < n; ++q) {
-                const float dx = d->xyz[3 * q] - d->xyz[3 * i], dy = d->xyz[3 * q + 1] - d->xyz[3 * i + 1],
-                            dz = d->xyz[3 * q + 2] - d->xyz[3 * i + 2];
-                if (!bonded[(size_t)i * n + q] && std::sqrt(dx * dx + dy * dy + dz * dz) < cut) total += 2;
-            }
-        int64_t want = (int64_t)std::ceil(1.10 * (double)total) + 4 * (int64_t)n;
-        want = std::min<int64_t>(want, (int64_t)n * h.cap_pl);
-        const int64_t fit =
-            ((int64_t)c->smem_dyn_max - (int64_t)resident_layout(n, h.ncov, h.nnat, h.bsm, 0).total - 16) / 2;
-        h.lcache = (int32_t)std::max<int64_t>(0, std::min(want, fit));
-    }
+    if (!h.grid) resident_shapes(c, d, m, std::min(p.pairlist_cutoff, p.pairs_threshold), h);
     if (h.grid) {
         h.lpb = kGridLpb;
         h.block = 1024;
@@ -1427,15 +1493,20 @@ extern "C" int sopb_job_create(sopb_context* c, const sopb_job_desc* d, sopb_job
     const size_t o_ex = o_natpar + align256(m.nat_par.size() * 8 + 8);
     const size_t o_ppm = o_ex + align256(mask_bytes);
     const size_t o_ppcnt = o_ppm + (h.mask ? align256(mask_bytes) : 0);
-    const size_t o_plcnt = o_ppcnt + align256((size_t)n * 4);
-    const size_t o_ppj = o_plcnt + align256((size_t)n * 4);
+    const size_t o_plcnt = o_ppcnt + (h.mask ? 0 : align256((size_t)n * 4));
+    // resident jobs: the Verlet rows of the pairs of beads and their headers,
+    // the near rows (pairs within pairlist_cutoff + skin) and the coordinates
+    // these were built at; grid jobs: index rows per bead
+    const int32_t np = job_pairs(n);
+    h.cap_u = h.mask ? (int32_t)row_cap(n, h.cap_pl, 2) : 0;
+    h.cap_nr = h.mask ? (int32_t)row_cap(n, h.cap_pl, 4) : 0;
+    const size_t o_vh = o_plcnt + (h.mask ? 0 : align256((size_t)n * 4));
+    const size_t o_ppj = o_vh + (h.mask ? align256((size_t)np * 8) : 0);
     const size_t o_plj = o_ppj + (h.mask ? 0 : align256((size_t)n * h.cap_pp * 4));
-    // resident jobs: the near list (pairs within pairlist_cutoff + skin,
-    // u16) and the coordinates it was built at
-    h.cap_nr = h.mask ? std::max<int32_t>(1, std::min<int32_t>(n - 1, 2 * h.cap_pl)) : 0;
-    const size_t o_nrj = o_plj + align256((size_t)n * h.cap_pl * 4);
-    const size_t o_nrc = o_nrj + (h.mask ? align256((size_t)n * h.cap_nr * 2) : 0);
-    const size_t o_xref = o_nrc + (h.mask ? align256((size_t)n * 4) : 0);
+    const size_t o_vr = o_plj + (h.mask ? 0 : align256((size_t)n * h.cap_pl * 4));
+    const size_t o_nrj = o_vr + (h.mask ? align256((size_t)np * h.cap_u * 2) : 0);
+    const size_t o_nrc = o_nrj + (h.mask ? align256((size_t)np * h.cap_nr * 2) : 0);
+    const size_t o_xref = o_nrc + (h.mask ? align256((size_t)np * 4) : 0);
     const size_t o_log = o_xref + (h.mask ? align256((size_t)n * 16) : 0);
     // event-log ring of the jobs whose updaters print per-update lines
     h.log_cap = (h.ramp || h.indent || h.plane) ? (p.log_rows > 0 ? p.log_rows : 1024) : 0;
@@ -1467,10 +1538,12 @@ extern "C" int sopb_job_create(sopb_context* c, const sopb_job_desc* d, sopb_job
     h.nat_par = (float2*)(base + o_natpar);
     h.ex_mask = h.grid ? nullptr : (uint32_t*)(base + o_ex);
     h.pp_mask = h.mask ? (uint32_t*)(base + o_ppm) : nullptr;
-    h.pp_cnt = (int32_t*)(base + o_ppcnt);
-    h.pl_cnt = (int32_t*)(base + o_plcnt);
+    h.pp_cnt = h.mask ? nullptr : (int32_t*)(base + o_ppcnt);
+    h.pl_cnt = h.mask ? nullptr : (int32_t*)(base + o_plcnt);
     h.pp_j = h.mask ? nullptr : (int32_t*)(base + o_ppj);
-    h.pl_j = (int32_t*)(base + o_plj);
+    h.pl_j = h.mask ? nullptr : (int32_t*)(base + o_plj);
+    h.vh = h.mask ? (uint2*)(base + o_vh) : nullptr;
+    h.vr = h.mask ? (uint16_t*)(base + o_vr) : nullptr;
     h.nr_j = h.mask ? (uint16_t*)(base + o_nrj) : nullptr;
     h.nr_cnt = h.mask ? (int32_t*)(base + o_nrc) : nullptr;
     h.x_ref = h.mask ? (float4*)(base + o_xref) : nullptr;
@@ -1491,7 +1564,7 @@ extern "C" int sopb_job_create(sopb_context* c, const sopb_job_desc* d, sopb_job
     h.tipF = c->tipF + b0;
     h.flags = c->flags + b0;
     cudaStream_t st = c->upload;   // set-up copies do not wait for running work
-    CUDA_TRY(cudaMemsetAsync(base + o_ppm, 0, o_ppj - o_ppm, st));   // mask and counts
+    CUDA_TRY(cudaMemsetAsync(base + o_ppm, 0, o_ppj - o_ppm, st));   // mask, counts and row headers
     if (!h.grid) CUDA_TRY(cudaMemcpyAsync(h.ex_mask, ex.data(), mask_bytes, cudaMemcpyHostToDevice, st));
     CUDA_TRY(cudaMemcpyAsync(h.cov_off, m.cov_off.data(), (n + 1) * 4, cudaMemcpyHostToDevice, st));
     if (!m.cov_j.empty()) {
@@ -1578,23 +1651,79 @@ namespace {
 // registers (the kernel's launch bound) and the SM's shared memory.
 int ctas_per_sm(const sopb_context* c, int block, size_t smem) {
     const int by_regs = 1024 / block;
-    const size_t per_cta = smem + (size_t)c->smem_static[block_index(block)] + (size_t)c->smem_reserved;
+    const size_t per_cta = smem + (size_t)c->smem_static + (size_t)c->smem_reserved;
     const int by_smem = (int)((size_t)c->smem_per_sm / per_cta);
     return std::max(1, std::min(by_regs, by_smem));
 }
-// Jobs of one class share a CTA size and the number of CTAs an SM holds, so
-// the class's largest shared-memory request never lowers the residency of
-// its smaller jobs.
+
+// CTAs per job of a run of resident jobs (log2, per job).  With one CTA per
+// job a run ends with its largest job, and one of fewer jobs than SMs leaves
+// SMs idle.  So the job that would take longest doubles its CTAs as long as
+// the run's CTAs have an SM each, within what clusters of that size reach,
+// or -- with enough jobs to fill the SMs anyway -- the job takes longer than
+// the run's work spread over all SMs (200 replicas of 60 to 600 beads: 3.0 ms
+// per 200 steps, 4.7 without); a CTA keeps at least kClusterMinBeads beads.  A step of n beads on C CTAs takes about
+// n / C bead times, plus the cluster's exchange, worth kClusterBeads beads
+// (200 steps of 600 beads: 3.5 ms on one CTA, 0.9 ms on sixteen).  A job's
+// arithmetic does not depend on its cluster.
+constexpr int kClusterMinBeads = 12;
+constexpr double kClusterBeads = 12.0;
+std::vector<int> cluster_sizes(const sopb_context* c, sopb_job* const* jobs, int32_t njobs) {
+    std::vector<int> lc((size_t)njobs, 0);
+    int64_t used = njobs;
+    double work = 0.0;
+    for (int32_t j = 0; j < njobs; ++j) work += jobs[j]->n;
+    auto cost = [&](int32_t j) { return (double)jobs[j]->n / (1 << lc[j]) + (lc[j] ? kClusterBeads : 0.0); };
+    for (;;) {
+        int32_t worst = 0;
+        for (int32_t j = 1; j < njobs; ++j)
+            if (cost(j) > cost(worst)) worst = j;
+        const int k = lc[worst];
+        if (k + 1 >= kClusterSizes || !c->cluster_ctas[k + 1] || (jobs[worst]->n >> (k + 1)) < kClusterMinBeads) return lc;
+        const bool one_wave = used + (1 << k) <= c->cluster_ctas[k + 1];
+        if (!one_wave && (k >= 2 || 5 * njobs < 4 * c->sm_count || cost(worst) < 1.15 * work / c->sm_count)) return lc;
+        lc[worst] = k + 1;
+        used += 1 << k;
+        work += kClusterBeads * (k ? 1 << k : 2);
+    }
+}
+
+// Jobs of one class share the lanes per bead, a cluster size, a CTA size and the number of CTAs
+// an SM holds, so the class's largest shared-memory request never lowers the
+// residency of its smaller jobs.
 void group_jobs(const sopb_context* c, sopb_job* const* jobs, int32_t njobs, std::vector<LaunchClass>& out) {
-    std::map<int, LaunchClass> cls;   // key: block * 64 + CTAs per SM
+    std::map<int, LaunchClass> cls;   // key: (lanes per bead, wide, cluster; CTA size, CTAs per SM)
     std::vector<int32_t> order(njobs);
     for (int32_t k = 0; k < njobs; ++k) order[k] = k;
     std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) { return jobs[a]->n > jobs[b]->n; });
+    const std::vector<int> lc = cluster_sizes(c, jobs, njobs);
     for (int32_t k : order) {
         const JobDev& h = jobs[k]->h;
-        const size_t smem = resident_smem_bytes(h);
-        LaunchClass& L = cls[h.block * 64 + ctas_per_sm(c, h.block, smem)];
-        L.block = h.block;
+        const int lg = lc[k], C = 1 << lg;
+        const size_t smem = resident_layout(h.n, C, h.lcov[lg], h.lnat[lg], h.bsm[lg], h.lcache[lg]).total;
+        // a CTA of a cluster: a warp per task of a step (pairs of beads, the
+        // noise of 32 beads) as far as they go, in wide lane groups if these
+        // still have a warp each
+        // One CTA: at most 512 threads where two such CTAs fit an SM's shared
+        // memory, so that their phases overlap (512 replicas of 60 to 600
+        // beads: 5.35 ms per 200 steps, 6.02 with 1024)
+        int block = h.block;
+        bool wide = false;
+        if (block == 1024 && ctas_per_sm(c, 512, smem) > 1) block = 512;
+        if (C > 1) {
+            const int nb = local_beads_max(h.n, C), np = (nb + 1) / 2, noise = (nb + 31) / 32, G = std::min(16, 2 * h.lpb);
+            wide = h.lpb == 4 && (np + 1) / 2 + noise <= kClusterBlock / 32;
+            const int per = 32 / (wide ? 2 * G : G);
+            block = 32 * std::min(kClusterBlock / 32, std::max(2, (np + per - 1) / per + noise));
+        }
+        // the CTAs of clusters have an SM each, so those of one size share a
+        // launch whatever their jobs' sizes (a launch per size would queue on
+        // the side streams)
+        LaunchClass& L = cls[((h.lpb * 2 + wide) * 8 + lg) * 4096 + (C > 1 ? 0 : block * 2 + ctas_per_sm(c, block, smem))];
+        L.block = std::max(L.block, block);
+        L.cluster = C;
+        L.lpb = h.lpb;
+        L.wide = wide;
         L.max_n = std::max(L.max_n, jobs[k]->n);
         L.smem = std::max(L.smem, smem);
         L.ids.push_back(jobs[k]->slot);
@@ -1691,7 +1820,7 @@ int run_ordered(sopb_context* c, sopb_job* const* jobs, int32_t njobs, const int
             CUDA_TRY(cudaMemcpyAsync(d_steps, steps.data(), steps.size() * 8, cudaMemcpyHostToDevice, st));
         }
         if (grid.empty() && cls.size() == 1)
-            return launch_resident(cls[0].block, (int)cls[0].ids.size(), cls[0].smem, st, c->d_jobs, d_ids, d_steps);
+            return launch_resident(cls[0], st, c->d_jobs, d_ids, d_steps);
     } else {
         // no resident jobs in this run: no classes to launch, and the table
         // on this stream is no longer the plan's
@@ -1711,8 +1840,7 @@ int run_ordered(sopb_context* c, sopb_job* const* jobs, int32_t njobs, const int
     for (size_t k = 0; k < cls.size(); ++k) {
         cudaStream_t s = f->side[k % kSideStreams];
         CUDA_TRY(cudaStreamWaitEvent(s, f->fork, 0));
-        rc = launch_resident(cls[k].block, (int)cls[k].ids.size(), cls[k].smem, s, c->d_jobs, d_ids + off[k],
-                             d_steps + off[k]);
+        rc = launch_resident(cls[k], s, c->d_jobs, d_ids + off[k], d_steps + off[k]);
         if (rc) return rc;
     }
     for (size_t g = 0; g < grid.size(); ++g) {
@@ -1923,6 +2051,27 @@ extern "C" int sopb_job_pairlist(sopb_job* j, int32_t possible, int32_t* counts,
                 }
             counts[i] = k;
             for (int32_t r = k; r < cap; ++r) rows[(size_t)i * cap + r] = -1;
+        }
+        return SOPB_OK;
+    }
+    if (j->h.mask) {
+        // a resident job's rows are kept per pair of beads: both beads'
+        // partners, then each bead's own, merged in increasing j
+        const int32_t np = job_pairs(n), cap_u = j->h.cap_u;
+        std::vector<uint2> vh(np);
+        std::vector<uint16_t> vr((size_t)np * cap_u);
+        CUDA_TRY(cudaMemcpyAsync(vh.data(), j->h.vh, vh.size() * sizeof(uint2), cudaMemcpyDeviceToHost, c->io));
+        CUDA_TRY(cudaMemcpyAsync(vr.data(), j->h.vr, vr.size() * 2, cudaMemcpyDeviceToHost, c->io));
+        SOPB_TRY(io_end(j, false));
+        std::vector<int32_t> row;
+        for (int32_t i = 0; i < n; ++i) {
+            const int nf = vh[i >> 1].y & 0xffff, n0 = vh[i >> 1].y >> 16, n1 = vh[i >> 1].x >> 20;
+            const uint16_t* r = vr.data() + (size_t)(i >> 1) * cap_u;
+            const uint16_t* own = r + nf + ((i & 1) ? n0 : 0);
+            row.resize((size_t)nf + ((i & 1) ? n1 : n0));
+            std::merge(r, r + nf, own, own + ((i & 1) ? n1 : n0), row.begin());
+            counts[i] = (int32_t)row.size();
+            for (int32_t k = 0; k < cap; ++k) rows[(size_t)i * cap + k] = k < (int32_t)row.size() ? row[k] >> 4 : -1;
         }
         return SOPB_OK;
     }

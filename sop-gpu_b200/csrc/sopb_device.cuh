@@ -17,6 +17,8 @@
 namespace sopb {
 
 enum : int { FLAG_FREE = 0, FLAG_FIXED = 1, FLAG_PULLED = 2 };
+constexpr int kMaxResidentBeads = 2048;
+constexpr int kClusterSizes = 5;   // CTAs of a resident job's cluster: 1, 2, 4, 8, 16
 constexpr int SOPB_STATUS_CAPACITY = SOPB_ERR_CAPACITY;
 constexpr int SOPB_STATUS_NONFINITE = SOPB_ERR_NONFINITE;
 
@@ -32,9 +34,10 @@ struct JobDev {
     int32_t max_pp;       // configured max_possiblePairs (overflow -> error)
     int32_t max_pl;       // configured max_pairs
     int32_t grid;         // 1: grid path (per-step kernels, CUDA graphs)
-    int32_t lcache;       // shared-memory cache of the Verlet list, entries
-    int32_t bsm;          // 1: bonded maps copied to shared memory for a launch
-    int32_t ncov, nnat;   // covalent / native map entries (both directions)
+    // resident launches, by log2 of the CTAs per job: entries of the shared
+    // Verlet rows, 1 when the bonded maps are copied to shared memory, and the
+    // most covalent / native map entries of one CTA's beads
+    int32_t lcache[kClusterSizes], bsm[kClusterSizes], lcov[kClusterSizes], lnat[kClusterSizes];
     int32_t stride;       // updater period (gsop.cu:117-122)
     int32_t nav;
     int32_t pairs_freq;
@@ -69,13 +72,16 @@ struct JobDev {
     float2* nat_par;      // (r0^2, -12 eh / r0^2)  (native.cu:112-146)
     int32_t* pp_cnt;      // [n]
     int32_t* pp_j;        // [n * cap_pp]
-    int32_t* pl_cnt;      // [n]
+    int32_t* pl_cnt;      // [n] Verlet rows of a grid job
     int32_t* pl_j;        // [n * cap_pl]
     uint32_t* ex_mask;    // [n * W] bonded + native partners and self
     uint32_t* pp_mask;    // [n * W] possible pairs (MASK mode)
-    uint16_t* nr_j;       // [n * cap_nr] near list: possible pairs within pairlist_cutoff + skin
-    int32_t* nr_cnt;      // [n]
+    uint2* vh;            // [ceil(n/2)] Verlet row headers of a resident job, per pair of beads
+    uint16_t* vr;         // [ceil(n/2) * cap_u] its rows: 16 j
+    uint16_t* nr_j;       // [ceil(n/2) * cap_nr] near rows: possible pairs within pairlist_cutoff + skin
+    int32_t* nr_cnt;      // [ceil(n/2)]
     float4* x_ref;        // coordinates the near list was built at
+    int32_t cap_u;        // row capacity of vr
     int32_t cap_nr;       // near-list row capacity
     int32_t nr_valid;     // 1: the near list holds every pair the next Verlet list can have
     float nr_t;           // r^2 threshold of the near list
@@ -170,14 +176,31 @@ __device__ __forceinline__ float dist2_rn(float4 xi, float4 xj) {
 }
 __device__ __forceinline__ bool within_cutoff(float4 xi, float4 xj, float t) { return dist2_rn(xi, xj) < t; }
 
-// FENE term (covalent_kernel.cu:28-51): Ks*(r-r0)/(r*(1-(r-r0)^2/R0^2)).
+// a / b for normal b and quotient: a reciprocal estimate refined by one
+// Newton step, then the quotient corrected by its residual (P. Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000
+// processor", 1990), within an ulp of the exact quotient.  It has no call and
+// no branch: a dependent chain of these takes about 45 cycles each where the
+// IEEE division (__fdiv_rn, a subroutine that handles every special operand)
+// takes 277.
+__device__ __forceinline__ float div_newton(float a, float b) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b));
+    r = fmaf(fmaf(-b, r, 1.0f), r, r);
+    const float q = a * r;
+    return fmaf(fmaf(-b, q, a), r, q);
+}
+
+// FENE term (covalent_kernel.cu:28-51): Ks*(r-r0)/(r*(1-(r-r0)^2/R0^2)),
+// numerator and denominator times R0^2 (one division).
 // r - r0 cancels for a near-relaxed bond, so r is formed with a correctly
 // rounded square root (the reference's fast-math build uses the approximate
 // one and loses ~1e-4 of the bond force there).
 __device__ __forceinline__ void fene_term(float4 xi, float4 xj, float r0, float ks, float R2, float3& f) {
     float dx = xj.x - xi.x, dy = xj.y - xi.y, dz = xj.z - xi.z;
-    float w = __fsqrt_rn(dx * dx + dy * dy + dz * dz) - r0;
-    w = __fdiv_rn(ks * w, (w + r0) * (1.0f - __fdiv_rn(w * w, R2)));
+    const float r = __fsqrt_rn(dx * dx + dy * dy + dz * dz);
+    float w = r - r0;
+    w = div_newton(ks * R2 * w, r * (R2 - w * w));
     f.x += w * dx;
     f.y += w * dy;
     f.z += w * dz;
@@ -185,7 +208,7 @@ __device__ __forceinline__ void fene_term(float4 xi, float4 xj, float r0, float 
 // Native LJ 12-6 term (native_kernel.cu:27-52).
 __device__ __forceinline__ void native_term(float4 xi, float4 xj, float2 par, float3& f) {
     float dx = xj.x - xi.x, dy = xj.y - xi.y, dz = xj.z - xi.z;
-    float w = par.x / (dx * dx + dy * dy + dz * dz);
+    float w = par.x * (1.0f / (dx * dx + dy * dy + dz * dz));
     float p6 = w * w * w;
     w = w * (p6 * p6 - p6) * par.y;
     f.x += dx * w;
@@ -205,6 +228,21 @@ __device__ __forceinline__ void pair_term(float4 xi, float4 xj, float c8, float 
     f.x += dx * w;
     f.y += dy * w;
     f.z += dz * w;
+}
+
+// The same term without the factor c8, which the caller applies to the sum:
+// d / r^8 within the cutoff.  (A resident bead's sum takes it once per row.)
+__device__ __forceinline__ void pair_term8(float4 xi, float4 xj, float cut2, float3& f) {
+    const float dx = xj.x - xi.x, dy = xj.y - xi.y, dz = xj.z - xi.z;
+    const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+    float w = 1.0f / r2;
+    w = w * w;
+    w = w * w;
+    if (r2 < cut2) {
+        f.x = fmaf(dx, w, f.x);
+        f.y = fmaf(dy, w, f.y);
+        f.z = fmaf(dz, w, f.z);
+    }
 }
 
 // Tip and continuous-surface terms (indentation_kernel.cu:71-128).  Returns

@@ -114,9 +114,9 @@ k_g_forces(JobDev* __restrict__ Jp, GridAux aux) {
         const float4 xi = J.x[act ? i : 0];
         float3 f = make_float3(0.f, 0.f, 0.f);
         if (act) {
-            bonded_partial(J, global_bonded(J), J.x, i, xi, l, lpb, f);
+            bonded_partial(J, J.x, i, xi, l, lpb, f);
             if ((J.cap_pl & 3) == 0) pair_row_v4(J, J.x, J.pl_j + (size_t)i * J.cap_pl, J.pl_cnt[i], xi, l, f);
-            else pairs_partial(J, J.x, nullptr, nullptr, 0, i, xi, l, lpb, f);
+            else pair_run(J, J.x, J.pl_j + (size_t)i * J.cap_pl, J.pl_cnt[i], xi, l, lpb, f);
             if (EXT && J.discrete) mica_partial(J, i, xi, l, lpb, f);
         }
         f = group_reduce(f, lpb);

@@ -66,16 +66,15 @@ k_obs_partial(const JobDev* __restrict__ Jp, double* __restrict__ part) {
                 if (dr < J.rlb || fabsf(sqrtf(par.x) - dr) <= R_limit) ++contacts;
             }
         }
-        const int32_t* row = J.pl_j + (size_t)i * J.cap_pl;
-        for (int k = 0; k < J.pl_cnt[i]; ++k) {
-            const float4 xj = J.x[row[k]];
+        for_partners(J, i, [&](int j) {
+            const float4 xj = J.x[j];
             const float dx = xj.x - xi.x, dy = xj.y - xi.y, dz = xj.z - xi.z;
             const float r2 = dx * dx + dy * dy + dz * dz;
             if (r2 < J.cut2) {
                 const float s = 1.0f / r2;
                 pairs += el_a6 * s * s * s;
             }
-        }
+        });
         v[0] += fene;
         v[1] += nat;
         v[2] += pairs;
