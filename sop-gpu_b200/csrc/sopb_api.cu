@@ -248,6 +248,13 @@ void hi_streams_destroy(sopb_job* j) {
     for (cudaEvent_t e : j->lk_ev) if (e) cudaEventDestroy(e);
 }
 
+// Most shared memory that k_hi_small asks for.
+int small_smem_max() {
+    int most = 0;
+    for (int n = 1; n <= 128; ++n) most = std::max(most, small_layout(n, small_ctas(n)).total);
+    return most * (int)sizeof(float);
+}
+
 // Opt a resident kernel in to the largest dynamic shared memory the device
 // allows next to the kernel's static shared memory.
 template <bool CL, bool WIDE, int G>
@@ -300,8 +307,8 @@ void launch_shape(const ShapePolicy& pol, int32_t n, int32_t lpb_req, int32_t* l
     *block = b;
 }
 
-// A resident launch of `njobs` jobs with `cluster` CTAs each.
-cudaLaunchConfig_t resident_config(int block, int cluster, int njobs, size_t smem, cudaStream_t st, cudaLaunchAttribute* at) {
+// A launch of `njobs` clusters of `cluster` CTAs each.
+cudaLaunchConfig_t cluster_config(int block, int cluster, int njobs, size_t smem, cudaStream_t st, cudaLaunchAttribute* at) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(njobs * cluster));
     cfg.blockDim = dim3((unsigned)block);
@@ -325,7 +332,7 @@ ResidentKernel resident_kernel(const LaunchClass& L) {
 
 int launch_resident(const LaunchClass& L, cudaStream_t st, JobDev* jobs, const int32_t* ids, const int64_t* steps) {
     cudaLaunchAttribute at;
-    const cudaLaunchConfig_t cfg = resident_config(L.block, L.cluster, (int)L.ids.size(), L.smem, st, &at);
+    const cudaLaunchConfig_t cfg = cluster_config(L.block, L.cluster, (int)L.ids.size(), L.smem, st, &at);
     CUDA_TRY(cudaLaunchKernelEx(&cfg, resident_kernel(L), jobs, ids, steps));
     CUDA_TRY(cudaGetLastError());
     return SOPB_OK;
@@ -508,7 +515,7 @@ extern "C" int sopb_context_create(int32_t device, void* stream, sopb_context** 
     c->cluster_ctas[0] = c->sm_count;
     for (int k = 1; k < kClusterSizes; ++k) {
         cudaLaunchAttribute at;
-        const cudaLaunchConfig_t cfg = resident_config(kClusterBlock, 1 << k, 1, (size_t)c->smem_dyn_max, nullptr, &at);
+        const cudaLaunchConfig_t cfg = cluster_config(kClusterBlock, 1 << k, 1, (size_t)c->smem_dyn_max, nullptr, &at);
         int clusters = 0;
         if (cudaOccupancyMaxActiveClusters(&clusters, k_resident_steps<true, false, 8>, &cfg) != cudaSuccess) {
             cudaGetLastError();   // this size does not run here
@@ -519,7 +526,7 @@ extern "C" int sopb_context_create(int32_t device, void* stream, sopb_context** 
     CUDA_TRY(cudaDeviceGetAttribute(&c->smem_per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, device));
     CUDA_TRY(cudaFuncSetAttribute(k_chol_potrf64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPotrfSmem));
     CUDA_TRY(cudaFuncSetAttribute(k_chol_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem));
-    CUDA_TRY(cudaFuncSetAttribute(k_chol_factor_panels, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallSmem));
+    CUDA_TRY(cudaFuncSetAttribute(k_hi_small, cudaFuncAttributeMaxDynamicSharedMemorySize, small_smem_max()));
     CUDA_TRY(cudaFuncSetAttribute(k_chol_apply_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, kCholMaxBeads * 12));
     CUDA_TRY(cudaDeviceGetAttribute(&c->smem_reserved, cudaDevAttrReservedSharedMemoryPerBlock, device));
     *out = c;
@@ -1087,13 +1094,16 @@ int grid_launch(sopb_job* j, cudaStream_t st, bool updaters, int steps, int due 
             // the factor is refreshed every step (hi_refresh 1, the
             // reference) or at the updater boundaries due for it
             const bool refresh = j->h.hi_refresh <= 1 || (s == 0 && refresh_first);
-            k_hi_prepare<<<nb, kGridBlock, 0, st>>>(Jp, a);
-            if (j->n <= 128) {
+            if (j->n > 128 || j->h.hi_bmode == SOPB_HI_B_REFCOMPAT) k_hi_prepare<<<nb, kGridBlock, 0, st>>>(Jp, a);
+            if (j->n <= 128 && j->h.hi_bmode == SOPB_HI_B_REFCOMPAT) {
                 k_chol_D<<<nb, kGridBlock, 0, st>>>(Jp, a, refresh ? 1 : 0);
-                if (refresh && j->h.hi_bmode == SOPB_HI_B_REFCOMPAT) k_chol_factor_small<<<1, 384, 0, st>>>(Jp, a);
-                else if (refresh) k_chol_factor_panels<<<1, kSmallThreads, kSmallSmem, st>>>(Jp, a);
-                if (j->h.hi_bmode == SOPB_HI_B_REFCOMPAT) k_chol_apply<<<nb, kGridBlock, 0, st>>>(Jp, a);
-                else k_chol_apply_warp<<<(j->n + kApplyWarps - 1) / kApplyWarps, 32 * kApplyWarps, 0, st>>>(Jp, a);
+                if (refresh) k_chol_factor_small<<<1, 384, 0, st>>>(Jp, a);
+                k_chol_apply<<<nb, kGridBlock, 0, st>>>(Jp, a);
+            } else if (j->n <= 128) {
+                cudaLaunchAttribute at;
+                const cudaLaunchConfig_t cfg = cluster_config(kSmallThreads, small_ctas(j->n), 1,
+                                                              small_layout(j->n, small_ctas(j->n)).total * sizeof(float), st, &at);
+                CUDA_TRY(cudaLaunchKernelEx(&cfg, k_hi_small, Jp, a, refresh ? 1 : 0));
             } else {
                 const dim3 tg((j->n + kHiTile - 1) / kHiTile, j->jsplit);
                 k_hi_df_partial<<<tg, kHiTile, 0, st>>>(Jp, a, j->jsplit);

@@ -10,12 +10,15 @@
 // reference's host does (src/Integrators/bdhitea.cu:133-176).
 //
 // Exact HI for jobs up to 128 beads (3n <= 384, the reference's CHOLSIZE,
-// src/Integrators/bdhitea.h:24): the normalised RPY tensor D is assembled
-// every step, factorised in place by one CTA per job (L below, L^T above
-// the diagonal, as integrateCholesky_decompose leaves it) and applied to the
-// random forces with either the true factor (B = L) or, for parity with the
-// reference, its symmetrised upper 3x3 blocks (integrateCholesky_L).
+// src/Integrators/bdhitea.h:24): the normalised RPY tensor D is assembled,
+// factorised and applied to the random forces by one cluster of CTAs
+// (k_hi_small, B = L); or, for parity with the reference's noise matrix, by
+// its own algorithm (L below, L^T above the diagonal, as
+// integrateCholesky_decompose leaves it) and its symmetrised upper 3x3 blocks
+// (integrateCholesky_L).
 #pragma once
+
+#include <type_traits>
 
 #include "sopb_grid.cuh"
 
@@ -362,126 +365,9 @@ k_chol_factor_small(JobDev* __restrict__ Jp, GridAux aux) {
     }
 }
 
-// The true factor L of D at n <= 128 (B = L), the same factorisation as
-// integrateCholesky_decompose (bdhitea_kernel.cu:154-190) in another order:
-// right-looking in 32-column panels, in one CTA.  The panel (its rows from
-// the diagonal down, at most 384 x 32) is factorised column by column with
-// one thread per row holding the row in registers (IEEE square root and
-// division, two barriers per column); it is written back, and the lower
-// triangle of the trailing matrix takes the panel's rank-32 update from L2
-// in 4 x 4 register tiles.  Only the lower triangle is written (the
-// reference also mirrors the factor into the upper one, which its
-// symmetrised noise matrix reads; that mode keeps k_chol_factor_small).
-constexpr int kSmallPanel = 32;
-constexpr int kSmallThreads = 512;                        // at least kSmallRows: one thread per panel row
-constexpr int kSmallRows = 384;                            // 3n for n <= 128
-constexpr int kSmallLd = kSmallPanel + 1;                  // floats per panel row in shared memory
-constexpr size_t kSmallSmem = (size_t)kSmallRows * kSmallLd * sizeof(float);
-static_assert(kSmallThreads >= kSmallRows, "one thread per panel row");
-
-__global__ void __launch_bounds__(kSmallThreads)
-k_chol_factor_panels(JobDev* __restrict__ Jp, GridAux aux) {
-    extern __shared__ float P[];                           // [rows][kSmallLd]
-    __shared__ float diag[kSmallPanel];
-    __shared__ float col_s[kSmallRows];                    // the scaled column of the panel
-    __shared__ float piv_s;
-    if (Jp->status) return;
-    const int m = 3 * Jp->n, ld = aux.ld, tid = threadIdx.x;
-    float* M = aux.tensor;
-    for (int p0 = 0; p0 < m; p0 += kSmallPanel) {
-        const int pb = min(kSmallPanel, m - p0), rows = m - p0;
-        for (int e = tid; e < rows * kSmallPanel; e += kSmallThreads) {
-            const int r = e / kSmallPanel, c = e % kSmallPanel;
-            P[r * kSmallLd + c] = c < pb && c <= r ? M[(size_t)(p0 + r) * ld + p0 + c] : 0.f;
-        }
-        __syncthreads();
-        // the panel, column by column: thread r holds panel row r in
-        // registers; per column the pivot's owner publishes it, every row
-        // below scales its entry and publishes it, then updates its row
-        {
-            const int r = tid;
-            const bool own = r < rows;
-            float row[kSmallPanel];
-#pragma unroll
-            for (int k = 0; k < kSmallPanel; ++k) row[k] = own ? P[r * kSmallLd + k] : 0.f;
-#pragma unroll
-            for (int c = 0; c < kSmallPanel; ++c) {   // unrolled: row[] indices are constants
-                if (c < pb) {                           // the same for the whole CTA
-                    if (r == c) piv_s = row[c];
-                    __syncthreads();
-                    const float d = __fsqrt_rn(piv_s);
-                    float lrc = 0.f;
-                    if (r == c) diag[c] = d;
-                    if (r > c && own) {
-                        lrc = __fdiv_rn(row[c], d);
-                        row[c] = lrc;
-                        col_s[r] = lrc;
-                    }
-                    __syncthreads();
-                    if (r > c && own) {
-#pragma unroll
-                        for (int k = c + 1; k < kSmallPanel; ++k)
-                            if (k < pb && k <= r) row[k] -= lrc * col_s[k];
-                    }
-                }
-            }
-            __syncthreads();
-            if (own) {
-#pragma unroll
-                for (int k = 0; k < kSmallPanel; ++k) P[r * kSmallLd + k] = row[k];
-            }
-            __syncthreads();
-        }
-        for (int e = tid; e < rows * kSmallPanel; e += kSmallThreads) {
-            const int r = e / kSmallPanel, c = e % kSmallPanel;
-            if (c < pb && c <= r) M[(size_t)(p0 + r) * ld + p0 + c] = r == c ? diag[c] : P[r * kSmallLd + c];
-        }
-        // trailing lower triangle: A22 -= L21 L21^T, 4 x 4 tiles (ti >= tj),
-        // consecutive threads along a tile row
-        const int n2 = rows - pb, nt = (n2 + 3) / 4, ntiles = nt * (nt + 1) / 2;
-        for (int t = tid; t < ntiles; t += kSmallThreads) {
-            int ti = (int)((sqrtf(8.f * (float)t + 1.f) - 1.f) * 0.5f);
-            while (ti * (ti + 1) / 2 > t) --ti;
-            while ((ti + 1) * (ti + 2) / 2 <= t) ++ti;
-            const int tj = t - ti * (ti + 1) / 2;
-            float acc[4][4] = {};
-            const float* A = P + (size_t)(pb + 4 * ti) * kSmallLd;
-            const float* B = P + (size_t)(pb + 4 * tj) * kSmallLd;
-            for (int c = 0; c < pb; ++c) {
-                float a[4], b[4];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    a[u] = 4 * ti + u < n2 ? A[u * kSmallLd + c] : 0.f;
-                    b[u] = 4 * tj + u < n2 ? B[u * kSmallLd + c] : 0.f;
-                }
-#pragma unroll
-                for (int u = 0; u < 4; ++u)
-#pragma unroll
-                    for (int v = 0; v < 4; ++v) acc[u][v] += a[u] * b[v];
-            }
-            // all sixteen entries loaded before any is stored (one L2 round trip)
-            float mv[4][4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-#pragma unroll
-                for (int v = 0; v < 4; ++v) {
-                    const int row = 4 * ti + u, col = 4 * tj + v;
-                    mv[u][v] = row < n2 && col <= row ? M[(size_t)(p0 + pb + row) * ld + p0 + pb + col] : 0.f;
-                }
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-#pragma unroll
-                for (int v = 0; v < 4; ++v) {
-                    const int row = 4 * ti + u, col = 4 * tj + v;
-                    if (row < n2 && col <= row) M[(size_t)(p0 + pb + row) * ld + p0 + pb + col] = mv[u][v] - acc[u][v];
-                }
-        }
-        __syncthreads();
-    }
-}
-
-// integrateCholesky_L (bdhitea_kernel.cu:303-361): f_i = (D F)_i + sum_{q<=i}
-// B_iq (rho g)_q, then the fixed beads and the Ermak-McCammon move.
+// integrateCholesky_L (bdhitea_kernel.cu:303-361) with the reference's noise
+// matrix: f_i = (D F)_i + sum_{q<=i} B_iq (rho g)_q, B the symmetrised upper
+// 3x3 blocks, then the fixed beads and the Ermak-McCammon move.
 __global__ void __launch_bounds__(kGridBlock)
 k_chol_apply(JobDev* __restrict__ Jp, GridAux aux) {
     const JobDev& J = *Jp;
@@ -493,24 +379,11 @@ k_chol_apply(JobDev* __restrict__ Jp, GridAux aux) {
         float3 f = make_float3(dfi.x, dfi.y, dfi.z);
         for (int q = 0; q <= i; ++q) {
             const float4 g = aux.rf[q];
-            if (J.hi_bmode == SOPB_HI_B_REFCOMPAT) {
-                const float* L0 = M + (size_t)(3 * q) * ld + 3 * i;
-                const float bxx = L0[0], bxy = L0[1], bxz = L0[2], byy = L0[ld + 1], byz = L0[ld + 2], bzz = L0[2 * ld + 2];
-                f.x += bxx * g.x + bxy * g.y + bxz * g.z;
-                f.y += bxy * g.x + byy * g.y + byz * g.z;
-                f.z += bxz * g.x + byz * g.y + bzz * g.z;
-            } else {
-                const float gg[3] = {g.x, g.y, g.z};
-                float acc[3];
-                for (int r = 0; r < 3; ++r) {
-                    acc[r] = 0.f;
-                    for (int c = 0; c < 3; ++c)
-                        if (3 * q + c <= 3 * i + r) acc[r] += M[(size_t)(3 * i + r) * ld + 3 * q + c] * gg[c];
-                }
-                f.x += acc[0];
-                f.y += acc[1];
-                f.z += acc[2];
-            }
+            const float* L0 = M + (size_t)(3 * q) * ld + 3 * i;
+            const float bxx = L0[0], bxy = L0[1], bxz = L0[2], byy = L0[ld + 1], byz = L0[ld + 2], bzz = L0[2 * ld + 2];
+            f.x += bxx * g.x + bxy * g.y + bxz * g.z;
+            f.y += bxy * g.x + byy * g.y + byz * g.z;
+            f.z += bxz * g.x + byz * g.y + bzz * g.z;
         }
         if (J.pulling && J.flags[i] == FLAG_FIXED) f = make_float3(0.f, 0.f, 0.f);
         const float4 xc = aux.xc[i];
@@ -520,46 +393,366 @@ k_chol_apply(JobDev* __restrict__ Jp, GridAux aux) {
     }
 }
 
-// integrateCholesky_L (bdhitea_kernel.cu:303-361) with the true factor at
-// n <= 128: a warp per bead; the lanes split the columns of the bead's three
-// rows of L (the noise vector rho g staged flat in shared memory), a fixed
-// xor-shuffle tree sums them, then (D F)_i, the fixed beads and the
-// Ermak-McCammon move as in k_chol_apply.
-constexpr int kApplyWarps = 8;
-__global__ void __launch_bounds__(32 * kApplyWarps)
-k_chol_apply_warp(JobDev* __restrict__ Jp, GridAux aux) {
-    __shared__ float gs[kSmallRows];
+// ---- exact HI with the true factor (B = L), n <= 128: one kernel per step --------
+// integrateTea_prepare, integrateCholesky_D, _decompose and _L
+// (bdhitea_kernel.cu:33-65, 89-190, 303-361) in one cluster of up to eight
+// CTAs that holds the 3n x 3n matrix in shared memory from its assembly to
+// the product with the noise.
+//   Rows are dealt to the CTAs in blocks of 32 (block b to CTA b mod C).
+//   Right-looking in panels of 32 columns: four warps of the diagonal block's
+//   owner factor the 32 x 32 tile (in registers, four lanes per row; its 8 x 8
+//   blocks by every lane for itself, so nothing but arithmetic sits between
+//   their pivots) and send the tile to every CTA; each CTA solves its rows
+//   below (four lanes per row) and sends them; each updates its own trailing
+//   tiles (a warp per 32 x 32 tile, a row per lane).  The next diagonal tile is
+//   updated first, by eight of its owner's warps, and factored while the other
+//   warps update the rest.
+//   All in FP32; a pivot's reciprocal root is an estimate with one Newton step,
+//   the root and the quotients by it are corrected by their residuals.
+// Then D F (a warp per bead), L g (a warp per row), the fixed beads and the
+// Ermak-McCammon move.  Between refreshes L is read from the tensor.
+// Bound: the serial chain of 3n/32 panels (factor 9000 cycles, solve and send
+// 5000, two cluster barriers).  90 beads, a new factor every step: 80 us a
+// step with the forces, 231 us with a one-CTA factor that kept the matrix in
+// L2 and took two barriers per column.
+constexpr int kSmallPanel = 32;
+constexpr int kSmallThreads = 512;
+constexpr int kSmallRows = 384;                            // 3n for n <= 128
+constexpr int kSmallMaxCtas = 8;
+constexpr int kSmallLdp = kSmallPanel + 4;                 // floats: rows of a panel, 16-byte aligned, no bank conflicts
+struct SmallLayout {                                       // in floats
+    int ldr, rows, P, Dg, dinv, S, x, mf, df, sd, g, total;
+};
+__host__ __device__ inline int small_blocks(int n) { return (3 * n + kSmallPanel - 1) / kSmallPanel; }
+__host__ __device__ inline int small_ctas(int n) {
+    const int T = small_blocks(n);
+    return T >= 8 ? 8 : (T >= 4 ? 4 : (T >= 2 ? 2 : 1));
+}
+__host__ __device__ inline SmallLayout small_layout(int n, int C) {
+    const int T = small_blocks(n), mp = kSmallPanel * T;
+    SmallLayout L;
+    L.ldr = mp + 4;
+    int o = 0;
+    L.rows = o; o += (T + C - 1) / C * kSmallPanel * L.ldr;
+    L.P = o;    o += mp * kSmallLdp;
+    L.Dg = o;   o += kSmallPanel * kSmallLdp;
+    L.dinv = o; o += kSmallPanel;
+    L.S = o;    o += 64;
+    L.x = o;    o += 4 * n;
+    L.mf = o;   o += 4 * n;
+    L.df = o;   o += 4 * n;
+    L.sd = o;   o += 4 * n;
+    L.g = o;    o += mp;
+    L.total = o;
+    return L;
+}
+
+// 1 / sqrt(p): the hardware estimate and one Newton-Raphson step; d = sqrt(p)
+// by one residual correction.
+__device__ __forceinline__ float rsqrt_newton(float p, float& d) {
+    float y = rsqrtf(p);
+    y = fmaf(0.5f * y, fmaf(-p * y, y, 1.0f), y);
+    d = p * y;
+    d = fmaf(fmaf(-d, d, p), 0.5f * y, d);
+    return y;
+}
+// a / d from r ~ 1 / d, corrected by the quotient's residual
+__device__ __forceinline__ float quotient(float a, float d, float r) {
+    const float q = a * r;
+    return fmaf(fmaf(-q, d, a), r, q);
+}
+
+__device__ __forceinline__ void load8(const float* p, float (&v)[8]) {
+    const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+    v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+// A row's eight entries of a lower-triangular solve against the 8 x 8 factor
+// block d8: x L^T = a.
+__device__ __forceinline__ void solve8(float (&a)[8], const float (&d8)[8][8], const float (&dinv)[8]) {
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+        float v = a[c];
+#pragma unroll
+        for (int q = 0; q < c; ++q) v = fmaf(-a[q], d8[c][q], v);
+        a[c] = quotient(v, d8[c][c], dinv[c]);
+    }
+}
+// a[k] -= x . l_k, l_k the eight entries at L + k kSmallLdp
+__device__ __forceinline__ void rank8(float (&a)[8], const float (&x)[8], const float* L) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        float l[8];
+        load8(L + k * kSmallLdp, l);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) a[k] = fmaf(-x[c], l[c], a[k]);
+    }
+}
+__device__ __forceinline__ void store8(float* p, const float (&v)[8]) {
+    *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+    *reinterpret_cast<float4*>(p + 4) = make_float4(v[4], v[5], v[6], v[7]);
+}
+__device__ __forceinline__ void send8(uint32_t addr, const float (&v)[8]) {
+    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]) : "memory");
+    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr + 16), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
+                 : "memory");
+}
+
+// A warp's eight rows, four lanes per row: lane 8 t + r holds entries 8 t ..
+// 8 t + 7 of row r (so a step's chain is eight entries long, not 32).  Both
+// functions walk the 8-column blocks s: the lanes t = s solve, hand the result
+// to the row's other lanes, and those beyond s take it off their entries.
+
+// Rows below the diagonal tile, solved against it (Dg, dinv).
+__device__ __forceinline__ void small_solve(float (&a)[8], const float* Dg, const float* dinv) {
+    const int lane = threadIdx.x & 31, t = lane >> 3, r = lane & 7;
+    for (int s = 0; s < kSmallPanel / 8; ++s) {
+        if (t == s) {
+            float d8[8][8], r8[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) load8(Dg + (8 * s + i) * kSmallLdp + 8 * s, d8[i]);
+            load8(dinv + 8 * s, r8);
+            solve8(a, d8, r8);
+        }
+        __syncwarp();
+        float x[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) x[c] = __shfl_sync(0xffffffffu, a[c], 8 * s + r);
+        if (t > s) rank8(a, x, Dg + 8 * t * kSmallLdp + 8 * s);
+    }
+}
+
+// Factors the diagonal tile at `tile` (row stride ldr) with the CTA's first
+// four warps and sends it and its pivots' reciprocals to every CTA.  S: 8 x 8
+// floats of scratch.
+constexpr int kSmallDiagWarps = 4;
+__device__ __noinline__ void small_diag(float* tile, int ldr, float* Dg, float* dinv, float* S, int C, int rank) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, t = lane >> 3, r = lane & 7, row = 8 * w + r;
+    // the four warps' barrier: counted by threads (barrier, not bar, whose
+    // warps have to arrive converged), after the lanes of the branches above
+    auto sync = [] {
+        __syncwarp();
+        asm volatile("barrier.sync 1, 128;" ::: "memory");
+    };
+    float a[8];
+    load8(tile + row * ldr + 8 * t, a);
+    for (int s = 0; s < kSmallPanel / 8; ++s) {
+        if (w == s && t == s) store8(S + 8 * r, a);
+        sync();
+        if (t == s && w >= s) {
+            float d8[8][8], r8[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) load8(S + 8 * i, d8[i]);
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                float d;
+                r8[c] = rsqrt_newton(d8[c][c], d);
+                d8[c][c] = d;
+#pragma unroll
+                for (int i = c + 1; i < 8; ++i) d8[i][c] = quotient(d8[i][c], d, r8[c]);
+#pragma unroll
+                for (int i = c + 1; i < 8; ++i)
+#pragma unroll
+                    for (int k = c + 1; k <= i; ++k) d8[i][k] = fmaf(-d8[i][c], d8[k][c], d8[i][k]);
+            }
+            solve8(a, d8, r8);               // rows of the block itself get their rows of the factor
+            store8(Dg + row * kSmallLdp + 8 * s, a);
+            if (w == s && r == 0) store8(dinv + 8 * s, r8);
+        }
+        sync();
+        float x[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) x[c] = __shfl_sync(0xffffffffu, a[c], 8 * s + r);
+        if (t > s && t <= w) rank8(a, x, Dg + 8 * t * kSmallLdp + 8 * s);
+    }
+    store8(tile + row * ldr + 8 * t, a);
+    const uint32_t mine = (uint32_t)__cvta_generic_to_shared(Dg + row * kSmallLdp + 8 * t);
+    const uint32_t inv = (uint32_t)__cvta_generic_to_shared(dinv + 8 * r);
+    float v[8];
+    load8(dinv + 8 * (r & 3), v);
+    for (int k = 1; k < C; ++k) {
+        const uint32_t to = (uint32_t)((rank + k) % C);
+        if (t <= w) send8(map_rank(mine, to), a);
+        if (w == 0 && lane < kSmallPanel / 8) send8(map_rank(inv, to), v);
+    }
+}
+
+// Columns [32 cb + 4 j0, 32 cb + 4 j1) of the tile of 32 rows at `rows` (row 0 of it
+// is row 32 gb): minus the panel's rank-32 product, a row per lane.
+__device__ __forceinline__ void small_tile(float* rows, int ldr, const float* P, int gb, int cb, int j0, int j1) {
+    const int lane = threadIdx.x & 31;
+    float x[kSmallPanel];
+#pragma unroll
+    for (int q = 0; q < kSmallPanel; q += 8) {
+        float v[8];
+        load8(P + (kSmallPanel * gb + lane) * kSmallLdp + q, v);
+#pragma unroll
+        for (int t = 0; t < 8; ++t) x[q + t] = v[t];
+    }
+    for (int j = j0; j < j1; ++j) {
+        const float* p = P + (kSmallPanel * cb + 4 * j) * kSmallLdp;
+        float acc[4] = {};
+#pragma unroll
+        for (int q = 0; q < kSmallPanel; q += 4)
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                const float4 b = *reinterpret_cast<const float4*>(p + t * kSmallLdp + q);
+                acc[t] = fmaf(x[q], b.x, acc[t]);
+                acc[t] = fmaf(x[q + 1], b.y, acc[t]);
+                acc[t] = fmaf(x[q + 2], b.z, acc[t]);
+                acc[t] = fmaf(x[q + 3], b.w, acc[t]);
+            }
+        float4* dst = reinterpret_cast<float4*>(rows + lane * ldr + kSmallPanel * cb + 4 * j);
+        float4 v = *dst;
+        v.x -= acc[0];
+        v.y -= acc[1];
+        v.z -= acc[2];
+        v.w -= acc[3];
+        *dst = v;
+    }
+}
+
+__global__ void __launch_bounds__(kSmallThreads, 1)
+k_hi_small(JobDev* __restrict__ Jp, GridAux aux, int refresh) {
+    extern __shared__ __align__(16) float sm[];
     const JobDev& J = *Jp;
-    if (J.status) return;
-    const int n = J.n, ld = aux.ld, lane = threadIdx.x & 31;
-    for (int q = threadIdx.x; q < n; q += blockDim.x) {
-        const float4 g = aux.rf[q];
-        gs[3 * q] = g.x;
-        gs[3 * q + 1] = g.y;
-        gs[3 * q + 2] = g.z;
+    if (J.status) return;                                   // the same for the whole cluster
+    const int C = (int)cluster_nctarank(), rank = (int)cluster_ctarank();
+    const int n = J.n, m = 3 * n, T = small_blocks(n), ld = aux.ld;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr int kWarps = kSmallThreads / 32;
+    const SmallLayout lay = small_layout(n, C);
+    const int ldr = lay.ldr;
+    float *rows = sm + lay.rows, *P = sm + lay.P, *Dg = sm + lay.Dg, *dinv = sm + lay.dinv, *S = sm + lay.S, *g = sm + lay.g;
+    float4 *xs = reinterpret_cast<float4*>(sm + lay.x), *mf = reinterpret_cast<float4*>(sm + lay.mf),
+           *df = reinterpret_cast<float4*>(sm + lay.df);
+    uint4* sd = reinterpret_cast<uint4*>(sm + lay.sd);
+    // integrateTea_prepare (bdhitea_kernel.cu:33-65), by every CTA
+    for (int q = tid; q < n; q += kSmallThreads) {
+        xs[q] = J.x[q];
+        uint4 st = J.seeds[q];
+        const float4 gg = gaussian4(st);
+        sd[q] = st;
+        g[3 * q] = gg.x * J.var;
+        g[3 * q + 1] = gg.y * J.var;
+        g[3 * q + 2] = gg.z * J.var;
+        float4 f = aux.F[q];
+        if (J.pulling) {
+            const uint8_t fl = J.flags[q];
+            if (fl == FLAG_FIXED) f.x = f.y = f.z = 0.f;
+            if (fl == FLAG_PULLED) { f.x += J.pullF[0]; f.y += J.pullF[1]; f.z += J.pullF[2]; }
+        }
+        mf[q] = f;
     }
     __syncthreads();
-    const float* M = aux.tensor;
-    const int i = blockIdx.x * kApplyWarps + (threadIdx.x >> 5);
-    if (i >= n) return;
-    float acc[3];
+    const float a = J.hi_a;
+    float* M = aux.tensor;
+    if (refresh) {
+        // D's rows of this CTA, lower triangle; rows past 3n are the identity's
+        for (int lb = 0, gb = rank; gb < T; ++lb, gb += C) {
+            const int r0 = kSmallPanel * gb, i0 = r0 / 3, i1 = min(n - 1, (r0 + kSmallPanel - 1) / 3);
+            float* R = rows + lb * kSmallPanel * ldr;
+            for (int e = tid; e < (i1 - i0 + 1) * (i1 + 1); e += kSmallThreads) {
+                const int i = i0 + e / (i1 + 1), q = e % (i1 + 1);
+                if (q > i) continue;
+                Blk6 d{1.f, 0.f, 0.f, 1.f, 0.f, 1.f};
+                if (q < i) d = rpy_between(xs[i], xs[q], a);
+                const float b[3][3] = {{d.xx, d.xy, d.xz}, {d.xy, d.yy, d.yz}, {d.xz, d.yz, d.zz}};
 #pragma unroll
-    for (int r = 0; r < 3; ++r) {
-        const int row = 3 * i + r;
-        const float* Lr = M + (size_t)row * ld;
-        float a = 0.f;
-        for (int c = lane; c <= row; c += 32) a += Lr[c] * gs[c];
-        for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-        acc[r] = a;
+                for (int u = 0; u < 3; ++u) {
+                    const int r = 3 * i + u - r0;
+                    if (r >= 0 && r < kSmallPanel)
+#pragma unroll
+                        for (int v = 0; v < 3; ++v) R[r * ldr + 3 * q + v] = b[u][v];
+                }
+            }
+            for (int e = tid; e < (r0 + kSmallPanel - max(m, r0)) * (r0 + kSmallPanel); e += kSmallThreads) {
+                const int r = max(m, r0) + e / (r0 + kSmallPanel), c = e % (r0 + kSmallPanel);
+                R[(r - r0) * ldr + c] = r == c ? 1.f : 0.f;
+            }
+        }
+        __syncthreads();
+        if (rank == 0 && warp < kSmallDiagWarps) small_diag(rows, ldr, Dg, dinv, S, C, rank);
+        for (int p = 0; p < T; ++p) {
+            cluster_sync_all();                            // the factored tile is everywhere
+            const int lb0 = (p + C - rank) / C;            // this CTA's first block below p
+            const int nlb = (T - rank + C - 1) / C - lb0;  // and their number
+            for (int t = warp; t < kSmallPanel / 8 * nlb; t += kWarps) {
+                const int lb = lb0 + t / (kSmallPanel / 8), r = 8 * (t % (kSmallPanel / 8)) + (lane & 7), c = 8 * (lane >> 3);
+                float* src = rows + (lb * kSmallPanel + r) * ldr + kSmallPanel * p + c;
+                float x[8];
+                load8(src, x);
+                small_solve(x, Dg, dinv);
+                store8(src, x);
+                const uint32_t to =
+                    (uint32_t)__cvta_generic_to_shared(P + (kSmallPanel * (lb * C + rank) + r) * kSmallLdp + c);
+                for (int k = 0; k < C; ++k) send8(map_rank(to, (uint32_t)((rank + k) % C)), x);
+            }
+            cluster_sync_all();                            // the panel is everywhere
+            if (p + 1 == T) break;
+            const bool next = rank == (p + 1) % C;         // owner of the next diagonal tile
+            float* R1 = rows + (p + 1) / C * kSmallPanel * ldr;
+            if (next) {
+                if (warp < 8) small_tile(R1, ldr, P, p + 1, p + 1, warp, warp + 1);
+                __syncthreads();
+                if (warp < kSmallDiagWarps) small_diag(R1 + kSmallPanel * (p + 1), ldr, Dg, dinv, S, C, rank);
+            }
+            // the other tiles: block gb's columns p + 1 .. gb
+            if (!next || warp >= kSmallDiagWarps) {
+                int t = next ? warp - kSmallDiagWarps : warp;
+                for (int lb = lb0; lb < lb0 + nlb; ++lb) {
+                    const int gb = lb * C + rank, first = gb == p + 1 ? gb + 1 : p + 1;
+                    const int count = gb - first + 1;
+                    for (; t < count; t += next ? kWarps - kSmallDiagWarps : kWarps)
+                        small_tile(rows + lb * kSmallPanel * ldr, ldr, P, gb, first + t, 0, kSmallPanel / 4);
+                    t -= count;
+                }
+            }
+            __syncthreads();
+        }
+        for (int lb = 0, gb = rank; gb < T; ++lb, gb += C)
+            for (int r = warp; r < kSmallPanel; r += kWarps) {
+                const int gr = kSmallPanel * gb + r;
+                if (gr < m)
+                    for (int c = lane; c <= gr; c += 32) M[(size_t)gr * ld + c] = rows[(lb * kSmallPanel + r) * ldr + c];
+            }
     }
-    if (lane == 0) {
-        const float4 dfi = aux.F[i];
-        float3 f = make_float3(dfi.x + acc[0], dfi.y + acc[1], dfi.z + acc[2]);
+    // (L g)_r, a warp per row, and (D F)_i, a warp per bead
+    float* y = reinterpret_cast<float*>(aux.part);
+    for (int lb = 0, gb = rank; gb < T; ++lb, gb += C)
+        for (int r = warp; r < kSmallPanel; r += kWarps) {
+            const int gr = kSmallPanel * gb + r;
+            if (gr >= m) continue;
+            const float* Lr = refresh ? rows + (lb * kSmallPanel + r) * ldr : M + (size_t)gr * ld;
+            float s = 0.f;
+            for (int c = lane; c <= gr; c += 32) s = fmaf(Lr[c], g[c], s);
+            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            if (lane == 0) y[gr] = s;
+        }
+    for (int i = rank + C * warp; i < n; i += C * kWarps) {
+        const float4 xi = xs[i];
+        float3 f = make_float3(0.f, 0.f, 0.f);
+        for (int q = lane; q < n; q += 32)
+            if (q != i) {
+                const Blk6 d = rpy_fast(xi, xs[q], a, 1.f / a);
+                const float4 fq = mf[q];
+                f.x += d.xx * fq.x + d.xy * fq.y + d.xz * fq.z;
+                f.y += d.xy * fq.x + d.yy * fq.y + d.yz * fq.z;
+                f.z += d.xz * fq.x + d.yz * fq.y + d.zz * fq.z;
+            }
+        f = group_reduce(f, 32);
+        if (lane == 0) df[i] = make_float4(mf[i].x + f.x, mf[i].y + f.y, mf[i].z + f.z, 0.f);
+    }
+    __syncthreads();
+    cluster_sync_all();                                    // y is complete, every CTA has read the job's state
+    for (int i = rank + C * tid; i < n; i += C * kSmallThreads) {
+        float3 f = make_float3(df[i].x + __ldcg(y + 3 * i), df[i].y + __ldcg(y + 3 * i + 1), df[i].z + __ldcg(y + 3 * i + 2));
         if (J.pulling && J.flags[i] == FLAG_FIXED) f = make_float3(0.f, 0.f, 0.f);
-        const float4 xc = aux.xc[i];
+        const float4 xc = xs[i];
         const float dx = J.hOverZeta * f.x, dy = J.hOverZeta * f.y, dz = J.hOverZeta * f.z;
         J.x[i] = make_float4(xc.x + dx, xc.y + dy, xc.z + dz, xc.w);
         J.T[i] = J.T[i] + J.tempNorm * (dx * dx + dy * dy + dz * dz);
+        J.seeds[i] = sd[i];
     }
 }
 

@@ -513,7 +513,7 @@ __device__ __forceinline__ uint32_t cluster_nctarank() {
     return r;
 }
 __device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
 // The address of CTA `rank`'s copy of this CTA's shared address `a`.
 __device__ __forceinline__ uint32_t map_rank(uint32_t a, uint32_t rank) {
