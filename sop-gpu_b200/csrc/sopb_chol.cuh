@@ -70,284 +70,183 @@ k_hi_assemble(const JobDev* __restrict__ Jp, GridAux aux) {
     }
 }
 
-// Cholesky of the diagonal tile (J, J), nb <= 128 rows, and the inverse of
-// its factor, in FP64 in shared memory, one CTA of 512 threads.
-// Factor, by 8-wide sub-panels: every thread that solves a row factors the
-// sub-panel's 8 x 8 diagonal block in registers (the same arithmetic in each
-// thread, so nothing but a barrier sits between the pivots of a sub-panel;
-// one FP64 rsqrt per pivot gives both L_cc = d rsqrt(d) and 1 / L_cc),
-// solves its row of the sub-panel below the block (kept column-major beside
-// the tile as well); then the trailing lower triangle is updated by warps in
-// strips of 32 rows x 4 columns, a row per lane (eight terms per entry, in
-// column order).
-// Inverse X = L^-1 by recursive doubling: the sixteen 8 x 8 diagonal blocks
-// by forward substitution (a thread per column), then four levels that
-// merge pairs of diagonal blocks of size B = 8 .. 64, X_UT = -X_UU (L_UT
-// X_TT), two triangular products per level with all 512 threads (its
-// critical path is about 2B dependent FMAs per level instead of the 128 of
-// a forward substitution).  X's strict lower triangle is kept transposed in
-// the unused upper triangle of the tile, its diagonal beside it.  Tile loads
-// are issued unconditionally (clamped addresses), 32 per thread in flight.
-// Out: the factor (FP32) into the tensor's tile, X (FP32, zero above the
-// diagonal and outside nb) into the inverse buffer of J's parity (aux.linv
-// holds two) for the tile-column solves.  A
-// pivot that is not positive sets the job's status.
+// Cholesky of the diagonal tile (J, J), nb <= 128 rows, and the inverse X of
+// its factor, in FP64 in shared memory, one CTA of 512 threads.  The lower
+// triangle is 136 blocks of 8 x 8; sixteen steps k, each for block column k:
+//   eight warps factor the 8 x 8 diagonal block, every thread for itself in
+//     registers (nothing but arithmetic sits between its pivots), and with it
+//     solve, a thread per row, the rows below (L) and, a thread per column, the
+//     rows k of the inverse (X_k = L_kk^-1 (I - sum_{j<k} L_kj X_j)); both go to
+//     shared memory for the next part and to global memory as results;
+//   every block (I, J) of a row I > k takes one rank-8 product from the FP64
+//     matrix unit: -= L_Ik L_Jk^T while J > k (the factorisation), -= L_Ik X_kJ
+//     once J <= k (the inverse's right-hand side, which starts from zero in the
+//     place of the block of L that has just been read).
+// So the inverse needs no phase of its own: its products fill the same steps.
+// Out: the factor (FP32) into the tensor's tile and X into the inverse buffer
+// of J's parity (aux.linv holds two, zero above the diagonal from the start)
+// for the tile-column solves.  A pivot that is not positive sets the job's
+// status.
+// Bound: per step the chain of eight pivots (about 1200 cycles with the solve)
+// and the blocks' shared-memory traffic (16 wavefronts per block and step).
+// A tile takes 43 us (67 us as sub-panels with FMA updates and a separate
+// inverse); 601 beads, a new factor every 5 of 10 steps: 3.15 ms, was 3.86 ms.
 constexpr int kPotrfThreads = 512;
-constexpr int kPotrfW = 8;                    // sub-panel width
-constexpr int kPotrfLd = kCT + 1;             // doubles
-constexpr size_t kPotrfSmem = (size_t)(kCT * kPotrfLd + 2 * kCT + kPotrfW * kCT + kCT * kCT / 4) * sizeof(double);
+constexpr int kPotrfW = 8;                    // step width
+constexpr int kPotrfSteps = kCT / kPotrfW;
+constexpr int kPotrfLd = kCT + 8;             // doubles: two rows of a block fill the banks once
+constexpr int kPotrfLp = 12;                  // doubles per row of L's column: 8 rows x 4 hit every bank twice
+constexpr size_t kPotrfSmem = (size_t)(kCT * kPotrfLd + kCT * kPotrfLp + kPotrfW * kPotrfLd) * sizeof(double);
 
-// 1 / sqrt(d) in FP64 for d > 0: the FP32 estimate refined by two steps of
-// the Newton-Raphson iteration y <- y (3 - d y^2) / 2, each of which roughly
-// squares the relative error (2^-22 -> 2^-44 -> below FP64 rounding).
-__device__ __forceinline__ double rsqrt_nr(double d) {
-    double y = (double)rsqrtf((float)d);
-    y = y * (1.5 - 0.5 * d * y * y);
-    y = y * (1.5 - 0.5 * d * y * y);
-    return y;
+// 1 / sqrt(d) in FP64 for d > 0: the FP32 estimate y (relative error 2^-22)
+// and one third-order Householder step, y (1 + e / 2 + 3 e^2 / 8) with
+// e = 1 - d y^2, whose error is of order e^3.
+__device__ __forceinline__ double rsqrt_householder(double d) {
+    const double y = (double)rsqrtf((float)d);
+    const double e = fma(-d * y, y, 1.0);
+    return fma(y * e, fma(0.375, e, 0.5), y);
 }
 
-// rows c0 .. c0 + 7 of the sub-panel's diagonal block, factorised in registers
-__device__ __forceinline__ void diag8_factor(const double* P, int c0, int w, double (&d8)[kPotrfW][kPotrfW],
-                                             double (&rinv)[kPotrfW], int& bad) {
+// Factors the 8 x 8 diagonal block (rows of `P`, stride kPotrfLd) in registers
+// and solves L x = v on the way (a row's x L^T = v is the same arithmetic).
+__device__ __forceinline__ void diag8_solve(const double* P, double (&x)[kPotrfW], int& bad) {
+    double d8[kPotrfW][kPotrfW];
 #pragma unroll
     for (int i = 0; i < kPotrfW; ++i)
 #pragma unroll
-        for (int jj = 0; jj < kPotrfW; ++jj)
-            d8[i][jj] = (jj <= i && i < w) ? P[(c0 + i) * kPotrfLd + c0 + jj] : (i == jj ? 1.0 : 0.0);
+        for (int q = 0; q <= i; q += 2) {
+            const double2 v = *reinterpret_cast<const double2*>(P + i * kPotrfLd + q);
+            d8[i][q] = v.x;
+            if (q + 1 <= i) d8[i][q + 1] = v.y;
+        }
 #pragma unroll
     for (int c = 0; c < kPotrfW; ++c) {
         const double piv = d8[c][c];
-        if (c < w && !(piv > 0.0)) bad = 1;
-        const double rs = rsqrt_nr(piv);
-        d8[c][c] = piv * rs;
-        rinv[c] = rs;
+        if (!(piv > 0.0)) bad = 1;
+        const double rs = rsqrt_householder(piv);
 #pragma unroll
         for (int i = c + 1; i < kPotrfW; ++i) d8[i][c] *= rs;
 #pragma unroll
         for (int i = c + 1; i < kPotrfW; ++i)
 #pragma unroll
-            for (int jj = c + 1; jj <= i; ++jj) d8[i][jj] -= d8[i][c] * d8[jj][c];
+            for (int q = c + 1; q <= i; ++q) d8[i][q] = fma(-d8[i][c], d8[q][c], d8[i][q]);
+        x[c] *= rs;
+#pragma unroll
+        for (int i = c + 1; i < kPotrfW; ++i) x[i] = fma(-x[c], d8[i][c], x[i]);
     }
 }
 
-// One level of the recursive inverse: pairs of diagonal blocks of size B
-// (top T, bottom U) merge as X_UT = -X_UU (L_UT X_TT), two triangular
-// products.  Thread: row i of its pair's block, R = B / 8 consecutive
-// columns j0 ..; the rows vary fastest within a warp, so the row-dependent
-// operand is read row-parallel and the other one is a broadcast.  X[a][c],
-// a > c, at P64[c][a]; X[a][a] at xd[a].  Ends with a barrier.
-template <int B>
-__device__ __forceinline__ void inv_level(double* P64, double* xd, double* ybuf) {
-    constexpr int R = B / 8;
-    const int tid = threadIdx.x, i = tid % B, j0 = ((tid / B) % 8) * R, pr = tid / (8 * B);
-    const int i0 = 2 * B * pr;                 // the pair's first row / column
-    double* Y = ybuf + pr * B * B;             // L_UT X_TT of this pair, row-major
-    {
-        double y[R];
-#pragma unroll
-        for (int t = 0; t < R; ++t) y[t] = 0.0;
-        const double* Lr = P64 + (i0 + B + i) * kPotrfLd + i0;
-        // X_TT[k][j] is zero for k < j: the first R values of k are triangular
-#pragma unroll
-        for (int dk = 0; dk < R; ++dk) {
-            const int kk = j0 + dk;
-            const double a = Lr[kk];
-#pragma unroll
-            for (int t = 0; t <= dk; ++t) {
-                const int j = j0 + t;
-                y[t] += a * (t == dk ? xd[i0 + j] : P64[(i0 + j) * kPotrfLd + i0 + kk]);
-            }
-        }
-        for (int kk = j0 + R; kk < B; ++kk) {
-            const double a = Lr[kk];
-#pragma unroll
-            for (int t = 0; t < R; ++t) y[t] += a * P64[(i0 + j0 + t) * kPotrfLd + i0 + kk];
-        }
-#pragma unroll
-        for (int t = 0; t < R; ++t) Y[i * B + j0 + t] = y[t];
-    }
-    __syncthreads();
-    {
-        double x[R];
-#pragma unroll
-        for (int t = 0; t < R; ++t) x[t] = 0.0;
-        const int a = i0 + B + i;
-        for (int kk = 0; kk < i; ++kk) {
-            const double xuu = P64[(i0 + B + kk) * kPotrfLd + a];
-#pragma unroll
-            for (int t = 0; t < R; ++t) x[t] -= xuu * Y[kk * B + j0 + t];
-        }
-        const double xaa = xd[a];
-#pragma unroll
-        for (int t = 0; t < R; ++t) P64[(i0 + j0 + t) * kPotrfLd + a] = x[t] - xaa * Y[i * B + j0 + t];
-    }
-    __syncthreads();
+// c += a b on the FP64 matrix unit: 8 x 8 by 8 x 4 and 4 x 8.  Lane: row
+// lane / 4 of c, columns 2 (lane % 4) and + 1; a[lane / 4][lane % 4];
+// b[lane % 4][lane / 4].
+__device__ __forceinline__ void mma_f64(double2& c, double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                 : "+d"(c.x), "+d"(c.y)
+                 : "d"(a), "d"(b));
 }
 
-__global__ void __launch_bounds__(kPotrfThreads)
+__global__ void __launch_bounds__(kPotrfThreads, 1)
 k_chol_potrf64(JobDev* __restrict__ Jp, GridAux aux, int J) {
-    // [kCT][kPotrfLd] tile, the diagonal of X [kCT], 1 / L_cc [kCT], the
-    // current sub-panel column-major [kPotrfW][kCT], inverse products
-    extern __shared__ double P64[];
-    __shared__ int stop;
-    if (threadIdx.x == 0) stop = Jp->status;
-    __syncthreads();
-    if (stop) return;
-    double* xd = P64 + kCT * kPotrfLd;
-    double* rdiag = xd + kCT;
-    double* panel = rdiag + kCT;
-    double* ybuf = panel + kPotrfW * kCT;     // [kCT * kCT / 4]: the products of one inverse level
-    const int m = 3 * Jp->n, ld = aux.ld, k = J * kCT, nb = min(kCT, m - k);
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    constexpr int kPer = kCT * kCT / kPotrfThreads;     // tile entries per thread
-    float* M = aux.tensor + (size_t)k * ld + k;
+    extern __shared__ __align__(16) double P64[];   // [kCT][kPotrfLd] the blocks
+    if (Jp->status) return;                         // read by every thread before any writes it (the barriers below)
+    double* Lp = P64 + kCT * kPotrfLd;              // [kCT][kPotrfLp] column k of L
+    double* Xk = Lp + kCT * kPotrfLp;               // [kPotrfW][kPotrfLd] X's rows of step k
+    constexpr int kWarps = kPotrfThreads / 32, kPer = kCT * kCT / 4 / kPotrfThreads;
+    const int m = 3 * Jp->n, ld = aux.ld, base = J * kCT, nb = min(kCT, m - base);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, fr = lane >> 2, fc = lane & 3;
+    float* M = aux.tensor + (size_t)base * ld + base;
     float* xout = aux.linv + (size_t)(J & 1) * kCT * kCT;   // two buffers: a solve may still read J - 1's
     {
-        float v[kPer];
+        // four columns per load, all of a thread's in flight (the leading
+        // dimension is a multiple of 32: a load past nb stays inside the row);
+        // rows and columns from nb on are the identity's
+        float4 v[kPer];
 #pragma unroll
         for (int u = 0; u < kPer; ++u) {
-            const int e = tid + u * kPotrfThreads, r = min(e >> 7, nb - 1), c = min(e & (kCT - 1), nb - 1);
-            v[u] = M[(size_t)r * ld + c];
+            const int e = tid + u * kPotrfThreads, r = e >> 5, q = 4 * (e & 31);
+            v[u] = r < nb && q < nb ? *reinterpret_cast<const float4*>(M + (size_t)r * ld + q) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
 #pragma unroll
         for (int u = 0; u < kPer; ++u) {
-            const int e = tid + u * kPotrfThreads, r = e >> 7, c = e & (kCT - 1);
-            if (r < nb && c <= r) P64[r * kPotrfLd + c] = (double)v[u];
+            const int e = tid + u * kPotrfThreads, r = e >> 5, q = 4 * (e & 31);
+            double d[4] = {(double)v[u].x, (double)v[u].y, (double)v[u].z, (double)v[u].w};
+#pragma unroll
+            for (int t = 0; t < 4; ++t)
+                if (r >= nb || q + t >= nb) d[t] = r == q + t ? 1.0 : 0.0;
+            double2* dst = reinterpret_cast<double2*>(P64 + r * kPotrfLd + q);
+            dst[0] = make_double2(d[0], d[1]);
+            dst[1] = make_double2(d[2], d[3]);
         }
     }
     __syncthreads();
     int bad = 0;
-    // ---- factor ----
-    for (int c0 = 0; c0 < nb; c0 += kPotrfW) {
-        const int w = min(kPotrfW, nb - c0), t0 = c0 + w;
-        const int r = t0 + tid;              // this thread's row of the sub-panel below its block
-        if (tid == 0 || r < nb) {
-            double d8[kPotrfW][kPotrfW], rinv[kPotrfW];
-            diag8_factor(P64, c0, w, d8, rinv, bad);
-            if (tid == 0)
-#pragma unroll
-                for (int i = 0; i < kPotrfW; ++i) {
-#pragma unroll
-                    for (int jj = 0; jj <= i; ++jj)
-                        if (i < w) P64[(c0 + i) * kPotrfLd + c0 + jj] = d8[i][jj];
-                    if (i < w) rdiag[c0 + i] = rinv[i];
-                }
-            if (r < nb) {
-                double x[kPotrfW];
-#pragma unroll
-                for (int c = 0; c < kPotrfW; ++c) x[c] = c < w ? P64[r * kPotrfLd + c0 + c] : 0.0;
-#pragma unroll
-                for (int c = 0; c < kPotrfW; ++c) {
-                    double v = x[c];
-#pragma unroll
-                    for (int q = 0; q < c; ++q) v -= x[q] * d8[c][q];
-                    x[c] = v * rinv[c];
-                }
-#pragma unroll
-                for (int c = 0; c < kPotrfW; ++c)
-                    if (c < w) {
-                        P64[r * kPotrfLd + c0 + c] = x[c];
-                        panel[c * kCT + r] = x[c];
-                    }
-            }
-        }
-        __syncthreads();
-        // trailing lower triangle, rows and columns t0 .. nb - 1: a warp
-        // takes a strip of 32 rows (a row per lane) by 4 columns at a time,
-        // the sub-panel read column-major (each lane its row's value, the
-        // four columns' values as broadcasts); eight terms per entry in
-        // column order
-        const int R = nb - t0, nstrips = (R + 31) >> 5;
-        int ntasks = 0;
-        for (int st = 0; st < nstrips; ++st) ntasks += (min(R, 32 * st + 32) + 3) >> 2;
-        for (int task = warp; task < ntasks; task += kPotrfThreads / 32) {
-            int st = 0, g = task;
-            while (g >= ((min(R, 32 * st + 32) + 3) >> 2)) {
-                g -= (min(R, 32 * st + 32) + 3) >> 2;
-                ++st;
-            }
-            const int row = t0 + 32 * st + lane, q0 = t0 + 4 * g;
-            double acc[4];
-#pragma unroll
-            for (int v = 0; v < 4; ++v)
-                acc[v] = (row < nb && q0 + v <= row) ? P64[row * kPotrfLd + q0 + v] : 0.0;
-#pragma unroll
-            for (int c = 0; c < kPotrfW; ++c) {
-                if (c < w) {
-                    const double x = row < nb ? panel[c * kCT + row] : 0.0;
-                    const double2 y01 = *reinterpret_cast<const double2*>(panel + c * kCT + q0);
-                    const double2 y23 = *reinterpret_cast<const double2*>(panel + c * kCT + q0 + 2);
-                    acc[0] -= x * y01.x;
-                    acc[1] -= x * y01.y;
-                    acc[2] -= x * y23.x;
-                    acc[3] -= x * y23.y;
-                }
-            }
-#pragma unroll
-            for (int v = 0; v < 4; ++v)
-                if (row < nb && q0 + v <= row) P64[row * kPotrfLd + q0 + v] = acc[v];
-        }
-        __syncthreads();
-    }
-    // ---- inverse X = L^-1 by recursive doubling of diagonal blocks ----
-    // X[a][c], a > c, lives at P64[c][a]; X[a][a] at xd[a].  Rows and columns
-    // from nb to 127 are made the identity first, so every level is full.
-    for (int e = tid; e < (kCT - nb) * kCT; e += kPotrfThreads) {
-        const int r = nb + e / kCT, c = e % kCT;
-        if (c <= r) P64[r * kPotrfLd + c] = r == c ? 1.0 : 0.0;
-        if (c == 0) rdiag[r] = 1.0;
-    }
-    __syncthreads();
-    if (tid < kCT) {
-        // the sixteen 8 x 8 diagonal blocks: thread (block, column cc)
-        // solves L_bb x = e_cc by forward substitution
-        const int b0 = tid & ~(kPotrfW - 1), cc = tid & (kPotrfW - 1);
+    const int row = tid, col = tid - kCT;
+    for (int k = 0; k < kPotrfSteps; ++k) {
+        // thread: row `row` of block column k, or column `col` of X's rows
+        const bool mine = tid < kCT ? row >= 8 * k : col < 8 * k + 8;
         double x[kPotrfW];
+        if (warp < 2 * kCT / 32) {
+            if (tid < kCT) {
 #pragma unroll
-        for (int r = 0; r < kPotrfW; ++r) {
-            double v = r == cc ? 1.0 : 0.0;
-#pragma unroll
-            for (int q = 0; q < r; ++q)
-                if (q >= cc) v -= P64[(b0 + r) * kPotrfLd + b0 + q] * x[q];
-            x[r] = r < cc ? 0.0 : v * rdiag[b0 + r];
-        }
-#pragma unroll
-        for (int r = 0; r < kPotrfW; ++r) {
-            if (r == cc) xd[b0 + r] = x[r];
-            else if (r > cc) P64[(b0 + cc) * kPotrfLd + b0 + r] = x[r];
-        }
-    }
-    __syncthreads();
-    // merge pairs of diagonal blocks of size B = 8, 16, 32, 64
-    inv_level<8>(P64, xd, ybuf);
-    inv_level<16>(P64, xd, ybuf);
-    inv_level<32>(P64, xd, ybuf);
-    inv_level<64>(P64, xd, ybuf);
-    // out: the factor's rows (zero above the diagonal) and X, four columns
-    // per store; a chunk that would pass column nb - 1 of the last tile
-    // column (and reach the next row) is stored column by column
-#pragma unroll 4
-    for (int u = 0; u < kPer / 4; ++u) {
-        const int e = tid + u * kPotrfThreads, r = e >> 5, c = (e & 31) * 4;
-        float lv[4], xv[4];
-#pragma unroll
-        for (int t = 0; t < 4; ++t) {
-            const int q = c + t;
-            lv[t] = (r < nb && q <= r) ? (float)P64[r * kPotrfLd + q] : 0.f;
-            xv[t] = (r < nb && q < nb) ? (r == q ? (float)xd[r] : (r > q ? (float)P64[q * kPotrfLd + r] : 0.f)) : 0.f;
-        }
-        *reinterpret_cast<float4*>(xout + r * kCT + c) = make_float4(xv[0], xv[1], xv[2], xv[3]);
-        if (r < nb) {
-            float* dst = M + (size_t)r * ld + c;
-            if (c + 4 <= nb) {
-                *reinterpret_cast<float4*>(dst) = make_float4(lv[0], lv[1], lv[2], lv[3]);
+                for (int q = 0; q < kPotrfW; q += 2) {
+                    const double2 v = *reinterpret_cast<const double2*>(P64 + row * kPotrfLd + 8 * k + q);
+                    x[q] = v.x;
+                    x[q + 1] = v.y;
+                }
             } else {
 #pragma unroll
-                for (int t = 0; t < 4; ++t)
-                    if (c + t < nb) dst[t] = lv[t];
+                for (int q = 0; q < kPotrfW; ++q)
+                    x[q] = col >= 8 * k ? (col - 8 * k == q ? 1.0 : 0.0) : P64[(8 * k + q) * kPotrfLd + col];
+            }
+            // (the block's own rows get their rows of the factor)
+            if (__any_sync(0xffffffffu, mine)) diag8_solve(P64 + 8 * k * kPotrfLd + 8 * k, x, bad);
+            if (mine && tid < kCT) {
+#pragma unroll
+                for (int q = 0; q < kPotrfW; q += 2)
+                    *reinterpret_cast<double2*>(Lp + row * kPotrfLp + q) = make_double2(x[q], x[q + 1]);
+            } else if (mine) {
+#pragma unroll
+                for (int q = 0; q < kPotrfW; ++q) Xk[q * kPotrfLd + col] = x[q];
             }
         }
+        __syncthreads();                            // L's and X's parts of step k are there
+        if (mine && tid < kCT) {
+            float* dst = M + (size_t)row * ld + 8 * k;
+            if (row >= 8 * k + 8 && row < nb) {     // then 8 k + 8 <= nb
+                *reinterpret_cast<float4*>(dst) = make_float4((float)x[0], (float)x[1], (float)x[2], (float)x[3]);
+                *reinterpret_cast<float4*>(dst + 4) = make_float4((float)x[4], (float)x[5], (float)x[6], (float)x[7]);
+            } else if (row < nb) {
+#pragma unroll
+                for (int q = 0; q < kPotrfW; ++q)
+                    if (8 * k + q <= row) dst[q] = (float)x[q];
+            }
+        } else if (mine && tid < 2 * kCT) {
+#pragma unroll
+            for (int q = 0; q < kPotrfW; ++q) {
+                const int r = 8 * k + q;
+                if (col <= r) xout[r * kCT + col] = r < nb && col < nb ? (float)x[q] : 0.f;
+            }
+        }
+        // the blocks of the rows below, the last row first, dealt to the warps
+        int I = kPotrfSteps - 1, q = warp;
+        while (I > k) {
+            if (q > I) {
+                q -= I + 1;
+                --I;
+                continue;
+            }
+            const double* A = Lp + (8 * I + fr) * kPotrfLp + fc;
+            const double* B = q > k ? Lp + (8 * q + fr) * kPotrfLp + fc : Xk + fc * kPotrfLd + 8 * q + fr;
+            double2* C = reinterpret_cast<double2*>(P64 + (8 * I + fr) * kPotrfLd + 8 * q + 2 * fc);
+            double2 c = *C;
+            const double a0 = -A[0], a1 = -A[4], b0 = B[0], b1 = B[q > k ? 4 : 4 * kPotrfLd];
+            if (q == k) c = make_double2(0.0, 0.0);
+            mma_f64(c, a0, b0);
+            mma_f64(c, a1, b1);
+            *C = c;
+            q += kWarps;
+        }
+        __syncthreads();
     }
     if (bad) atomicMax(&Jp->status, SOPB_ERR_HI);
 }
