@@ -899,7 +899,7 @@ int grid_possible(sopb_job* j, JobDev* Jp, cudaStream_t st, int force) {
     k_cl_fill<<<nb, kGridBlock, 0, st>>>(Jp, a, force);
     k_cl_possible<<<warps_blocks, kGridBlock, 0, st>>>(Jp, a, force);
     const int sort_blocks = (int)std::min<int64_t>((j->n + 3) / 4, (int64_t)j->ctx->sm_count * 16);
-    k_cl_sort_rows<<<sort_blocks, 128, 4 * kSortCap * sizeof(int32_t), st>>>(Jp, force);
+    k_cl_sort_rows<<<sort_blocks, 128, 4 * (kSortCap / 32 * 33) * sizeof(int32_t), st>>>(Jp, force);
     CUDA_TRY(cudaGetLastError());
     return SOPB_OK;
 }

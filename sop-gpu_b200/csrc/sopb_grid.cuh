@@ -23,7 +23,7 @@ namespace sopb {
 constexpr int kGridBlock = 256;
 constexpr int kGridLpb = 4;
 constexpr int kCellMax = 1 << 22;
-constexpr int kSortCap = 2048;   // rows up to this length are sorted in shared memory
+constexpr int kSortCap = 2048;   // rows up to this length are sorted in registers
 
 struct GridAux {
     // per-bead buffers of the grid path
@@ -358,16 +358,24 @@ k_cl_bounds(JobDev* __restrict__ Jp, GridAux aux, int force) {
 
 // Cell geometry: cells no smaller than the threshold (slightly enlarged so a
 // pair closer than the threshold is never two cells apart), at most kCellMax.
+// One warp: its lanes share the partial bounds (13 us for 198000 beads; 113
+// when one thread read them all).
 __global__ void k_cl_geometry(JobDev* __restrict__ Jp, GridAux aux, int nparts, int force) {
     const JobDev& J = *Jp;
     const int64_t step = job_step(Jp);
-    if (threadIdx.x != 0 || J.status || (!force && (step % J.stride != 0 || step % J.pp_freq != 0))) return;
+    if (J.status || (!force && (step % J.stride != 0 || step % J.pp_freq != 0))) return;
     float mn[3] = {3.4e38f, 3.4e38f, 3.4e38f}, mx[3] = {-3.4e38f, -3.4e38f, -3.4e38f};
-    for (int b = 0; b < nparts; ++b) {
+    for (int b = threadIdx.x; b < nparts; b += 32) {
         const float4 a = aux.part[b], z = aux.part[nparts + b];
         mn[0] = fminf(mn[0], a.x); mn[1] = fminf(mn[1], a.y); mn[2] = fminf(mn[2], a.z);
         mx[0] = fmaxf(mx[0], z.x); mx[1] = fmaxf(mx[1], z.y); mx[2] = fmaxf(mx[2], z.z);
     }
+    for (int o = 16; o > 0; o >>= 1)
+        for (int c = 0; c < 3; ++c) {
+            mn[c] = fminf(mn[c], __shfl_xor_sync(0xffffffffu, mn[c], o));
+            mx[c] = fmaxf(mx[c], __shfl_xor_sync(0xffffffffu, mx[c], o));
+        }
+    if (threadIdx.x != 0) return;
     float size = J.pp_thr * 1.0001f + 1e-3f;
     int dims[3] = {1, 1, 1};
     bool ok = true;
@@ -456,7 +464,9 @@ k_cl_fill(JobDev* __restrict__ Jp, GridAux aux, int force) {
 }
 
 // Candidates from the 27 neighbouring cells with the exact test, appended
-// unordered; one warp per bead.
+// unordered; one warp per bead.  Cells side by side in x hold their beads in
+// one run of the array, so there are nine runs to walk (1.59 ms for the
+// 198000-bead shell, 1.87 cell by cell).
 __global__ void __launch_bounds__(kGridBlock)
 k_cl_possible(JobDev* __restrict__ Jp, GridAux aux, int force) {
     __shared__ JobDev Js;
@@ -481,29 +491,25 @@ k_cl_possible(JobDev* __restrict__ Jp, GridAux aux, int force) {
             for (int dy = -1; dy <= 1; ++dy) {
                 const int y = cy + dy;
                 if (y < 0 || y >= d1) continue;
-                for (int dx = -1; dx <= 1; ++dx) {
-                    const int x = cx + dx;
-                    if (x < 0 || x >= d0) continue;
-                    const int c = (z * d1 + y) * d0 + x;
-                    const int s0 = aux.cell_start[c], s1 = aux.cell_start[c + 1];
-                    for (int kb = s0; kb < s1; kb += 32) {
-                        const int k = kb + l;
-                        int q = -1;
-                        bool ok = false;
-                        if (k < s1) {
-                            q = aux.cell_beads[k];
-                            ok = q != i && within_cutoff(xi, J.x[q], J.pp_t);
-                            for (int t = c0; t < c1 && ok; ++t) ok = J.cov_j[t] != q;
-                            for (int t = n0; t < n1 && ok; ++t) ok = J.nat_j[t] != q;
-                        }
-                        const unsigned m = __ballot_sync(0xffffffffu, ok);
-                        if (ok) {
-                            const int pos = cnt + __popc(m & ((1u << l) - 1u));
-                            if (pos < J.cap_pp) row[pos] = q;
-                            else err = SOPB_STATUS_CAPACITY;
-                        }
-                        cnt += __popc(m);
+                const int c = (z * d1 + y) * d0;
+                const int s0 = aux.cell_start[c + max(cx - 1, 0)], s1 = aux.cell_start[c + min(cx + 1, d0 - 1) + 1];
+                for (int kb = s0; kb < s1; kb += 32) {
+                    const int k = kb + l;
+                    int q = -1;
+                    bool ok = false;
+                    if (k < s1) {
+                        q = aux.cell_beads[k];
+                        ok = q != i && within_cutoff(xi, J.x[q], J.pp_t);
+                        for (int t = c0; t < c1 && ok; ++t) ok = J.cov_j[t] != q;
+                        for (int t = n0; t < n1 && ok; ++t) ok = J.nat_j[t] != q;
                     }
+                    const unsigned m = __ballot_sync(0xffffffffu, ok);
+                    if (ok) {
+                        const int pos = cnt + __popc(m & ((1u << l) - 1u));
+                        if (pos < J.cap_pp) row[pos] = q;
+                        else err = SOPB_STATUS_CAPACITY;
+                    }
+                    cnt += __popc(m);
                 }
             }
         }
@@ -512,41 +518,95 @@ k_cl_possible(JobDev* __restrict__ Jp, GridAux aux, int force) {
     if (err) atomicMax(&Jp->status, err);
 }
 
+// Sorts 32 R keys of a warp, R to a lane, ascending in blocked order (lane l
+// ends with the ranks R l to R l + R - 1): Batcher's bitonic network in the
+// form whose every comparator points up, since each merge starts with the
+// mirrored partner.  Partners up to R - 1 apart are in the same lane.
+template <int R, int STRIDE>
+__device__ __forceinline__ void sort_strides(int32_t (&v)[R], int l) {
+    if constexpr (STRIDE >= R) {
+        const bool low = (l & (STRIDE / R)) == 0;
+#pragma unroll
+        for (int a = 0; a < R; ++a) {
+            const int32_t o = __shfl_xor_sync(0xffffffffu, v[a], STRIDE / R);
+            v[a] = low ? min(v[a], o) : max(v[a], o);
+        }
+    } else if constexpr (STRIDE > 0) {
+#pragma unroll
+        for (int a = 0; a < R; ++a)
+            if ((a & STRIDE) == 0) {
+                const int32_t lo = min(v[a], v[a | STRIDE]);
+                v[a | STRIDE] = max(v[a], v[a | STRIDE]);
+                v[a] = lo;
+            }
+    }
+    if constexpr (STRIDE > 1) sort_strides<R, STRIDE / 2>(v, l);
+}
+
+template <int R, int SIZE = 2>
+__device__ __forceinline__ void sort_keys(int32_t (&v)[R], int l) {
+    if constexpr (SIZE <= R) {
+#pragma unroll
+        for (int a = 0; a < R; ++a)
+            if ((a ^ (SIZE - 1)) > a) {
+                const int32_t lo = min(v[a], v[a ^ (SIZE - 1)]);
+                v[a ^ (SIZE - 1)] = max(v[a], v[a ^ (SIZE - 1)]);
+                v[a] = lo;
+            }
+    } else {
+        // the lane mirrored within SIZE / R lanes, the register from the other end
+        const bool low = (l & (SIZE / R >> 1)) == 0;
+#pragma unroll
+        for (int a = 0; a < R / 2; ++a) {
+            const int32_t oa = __shfl_xor_sync(0xffffffffu, v[R - 1 - a], SIZE / R - 1);
+            const int32_t ob = __shfl_xor_sync(0xffffffffu, v[a], SIZE / R - 1);
+            v[a] = low ? min(v[a], oa) : max(v[a], oa);
+            v[R - 1 - a] = low ? min(v[R - 1 - a], ob) : max(v[R - 1 - a], ob);
+        }
+    }
+    if constexpr (SIZE > 2) sort_strides<R, SIZE / 4>(v, l);
+    if constexpr (SIZE < 32 * R) sort_keys<R, SIZE * 2>(v, l);
+}
+
+template <int R>
+__device__ __forceinline__ void sort_row(int32_t* row, int cnt, int32_t* sb, int l) {
+    int32_t v[R];
+#pragma unroll
+    for (int a = 0; a < R; ++a) v[a] = 32 * a + l < cnt ? row[32 * a + l] : 0x7fffffff;
+    sort_keys(v, l);
+    // through shared memory (a word of padding in 32) back into rows of 32
+#pragma unroll
+    for (int a = 0; a < R; ++a) sb[R * l + a + ((R * l + a) >> 5)] = v[a];
+    __syncwarp();
+#pragma unroll
+    for (int a = 0; a < R; ++a)
+        if (32 * a + l < cnt) row[32 * a + l] = sb[33 * a + l];
+    __syncwarp();
+}
+
 // Sorts every possible-pairs row ascending (the brute-force order); one warp
-// per row, bitonic sort in shared memory for rows up to kSortCap entries,
-// odd-even transposition in place for longer rows.
-__global__ void __launch_bounds__(128)
+// per row: the keys in registers and the comparators as shuffles for rows up
+// to kSortCap entries, odd-even transposition in place for longer rows.
+// Bound by instruction issue: 1.33 ms for a 198000-bead shell (3 capsids of 60 x 1100
+// beads), 9.2 ms with the keys and every comparator in shared memory.  128
+// registers (16 warps per SM) cover the longest class without a spill.
+__global__ void __launch_bounds__(128, 4)
 k_cl_sort_rows(JobDev* __restrict__ Jp, int force) {
-    extern __shared__ int32_t buf[];   // 4 warps x kSortCap
+    extern __shared__ int32_t buf[];   // 4 warps x kSortCap / 32 * 33
     const JobDev& J = *Jp;
     const int64_t step = job_step(Jp);
     if (J.status || (!force && (step % J.stride != 0 || step % J.pp_freq != 0))) return;
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    int32_t* sb = buf + w * kSortCap;
+    int32_t* sb = buf + w * (kSortCap / 32 * 33);
     for (int i = blockIdx.x * 4 + w; i < J.n; i += gridDim.x * 4) {
         const int cnt = J.pp_cnt[i];
         int32_t* row = J.pp_j + (size_t)i * J.cap_pp;
-        if (cnt <= kSortCap) {
-            int len = 1;
-            while (len < cnt) len <<= 1;
-            for (int k = l; k < len; k += 32) sb[k] = k < cnt ? row[k] : 0x7fffffff;
-            __syncwarp();
-            for (int size = 2; size <= len; size <<= 1) {
-                for (int stride = size >> 1; stride > 0; stride >>= 1) {
-                    for (int k = l; k < len; k += 32) {
-                        const int p = k ^ stride;
-                        if (p > k) {
-                            const bool up = (k & size) == 0;
-                            const int32_t a = sb[k], b = sb[p];
-                            if ((a > b) == up) { sb[k] = b; sb[p] = a; }
-                        }
-                    }
-                    __syncwarp();
-                }
-            }
-            for (int k = l; k < cnt; k += 32) row[k] = sb[k];
-            __syncwarp();
-        } else {
+        if (cnt <= 128) sort_row<4>(row, cnt, sb, l);
+        else if (cnt <= 256) sort_row<8>(row, cnt, sb, l);
+        else if (cnt <= 512) sort_row<16>(row, cnt, sb, l);
+        else if (cnt <= 1024) sort_row<32>(row, cnt, sb, l);
+        else if (cnt <= kSortCap) sort_row<64>(row, cnt, sb, l);
+        else {
             for (int pass = 0; pass < cnt; ++pass) {
                 for (int k = 2 * l + (pass & 1); k + 1 < cnt; k += 64) {
                     const int32_t a = row[k], b = row[k + 1];
@@ -557,6 +617,7 @@ k_cl_sort_rows(JobDev* __restrict__ Jp, int force) {
         }
     }
 }
+static_assert(kSortCap == 2048, "k_cl_sort_rows handles rows up to 32 x 64 keys in registers");
 
 // Near list of the Verlet rebuilds (a grid job with a skin): the possible
 // pairs within pairlist_cutoff + skin, in the order of the possible rows,
