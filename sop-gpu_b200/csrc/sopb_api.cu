@@ -750,7 +750,8 @@ struct GridLayout {
     bool cells = false, hi = false, exact = false, blocked = false;
     int plane_rows = 0, plane_ld = 0;
     size_t part = 0, rf = 0, mf = 0, xc = 0, ci = 0, eps = 0, ten = 0, linv = 0, phi = 0, plo = 0, geo = 0;
-    size_t cc = 0, cs = 0, cb = 0, bc = 0, near = 0, nrj = 0, nrc = 0, xref = 0;
+    size_t cc = 0, cs = 0, cb = 0, bc = 0, near = 0, nrj = 0, nrc = 0, xref = 0, vh = 0, vr = 0, vtot = 0;
+    int cap_u = 0, tile = 0;
     size_t total = 0;
 };
 
@@ -796,12 +797,25 @@ GridLayout grid_layout(const sopb_params& p, int64_t n, int sms, int64_t cap_pp,
         L.cb = take((size_t)n * 4);
         L.bc = take((size_t)n * 4);
     }
-    L.cap_nr = (int)grid_cap_nr(p, cap_pp, cap_pl);
+    // near rows: per bead with hydrodynamics; else per pair of beads, in the
+    // same bytes
+    const int64_t cap_nr = grid_cap_nr(p, cap_pp, cap_pl);
+    L.cap_nr = (int)(L.hi ? cap_nr : n * cap_nr / job_pairs((int)n));
     L.near = take(4 * sizeof(int32_t));
     if (L.cap_nr) {
-        L.nrj = take((size_t)n * L.cap_nr * 4);
+        L.nrj = take((size_t)n * cap_nr * 4);
         L.nrc = take((size_t)n * 4);
         L.xref = take((size_t)n * 16);
+    }
+    if (!L.hi) {
+        // rows per pair of beads: two Verlet rows' entries; tiles of a step's
+        // CTA (the last one whole)
+        L.tile = n <= kWideStepBeads ? 1 : step_pairs(false);
+        const int64_t tiles = (job_pairs((int)n) + L.tile - 1) / L.tile;
+        L.cap_u = (int)((row_cap(n, cap_pl, 2) + 3) & ~int64_t(3));
+        L.vh = take((size_t)job_pairs((int)n) * sizeof(int4));
+        L.vr = take((size_t)tiles * L.tile * L.cap_u * 4);
+        L.vtot = take((size_t)tiles * 4);
     }
     L.total = off;
     return L;
@@ -816,6 +830,7 @@ int grid_alloc(sopb_context* c, sopb_job* j, const sopb_params& p, int32_t n, in
     j->bead_blocks = L.npart;
     j->jsplit = L.jsplit;
     j->chol_w = c->policy.chol_panel_tiles;
+    a.n = n;
     a.npart = L.npart;
     a.use_cells = L.cells;
     a.cap_nr = L.cap_nr;
@@ -868,6 +883,13 @@ int grid_alloc(sopb_context* c, sopb_job* j, const sopb_params& p, int32_t n, in
         a.nr_j = (int32_t*)(b + L.nrj);
         a.nr_cnt = (int32_t*)(b + L.nrc);
         a.x_ref = (float4*)(b + L.xref);
+    }
+    if (!L.hi) {
+        a.vh = (int4*)(b + L.vh);
+        a.vr = (int32_t*)(b + L.vr);
+        a.vtot = (int32_t*)(b + L.vtot);
+        a.cap_u = L.cap_u;
+        a.tile = L.tile;
     }
     if (a.use_cells) {
         a.cell_count = (int32_t*)(b + L.cc);
@@ -1028,6 +1050,12 @@ int chol_refresh(sopb_job* j, JobDev* Jp, cudaStream_t st) {
     return SOPB_OK;
 }
 
+// CTAs of k_g_pair_rows: one per tile of pairs, as many as run at once.
+int pair_row_blocks(const sopb_job* j) {
+    const int group = std::max((int)j->aux.tile, kPairWarps);
+    return (int)std::min<int64_t>((job_pairs(j->n) + group - 1) / group, (int64_t)j->ctx->sm_count * 24);
+}
+
 // Updaters due at a stride boundary, from the host's copy of the step.  The
 // kernels of an updater that is not due return at once (each gates on the
 // device step itself); a launch sequence leaves them out.
@@ -1068,7 +1096,8 @@ int grid_launch(sopb_job* j, cudaStream_t st, bool updaters, int steps, int due 
         if (due & kDueVerlet) {
             const int wb = (int)std::min<int64_t>((j->n + 7) / 8, (int64_t)c->sm_count * 16);
             if (a.cap_nr) k_g_drift<<<nb, kGridBlock, 0, st>>>(Jp, a);
-            k_g_verlet<<<wb, kGridBlock, 0, st>>>(Jp, a, 0);
+            if (j->h.hi) k_g_verlet<<<wb, kGridBlock, 0, st>>>(Jp, a, 0);
+            else k_g_pair_rows<<<pair_row_blocks(j), 32 * kPairWarps, 0, st>>>(Jp, a, 0);
         }
         if (a.cap_nr && (due & (kDuePossible | kDueVerlet))) k_g_near_commit<<<1, 32, 0, st>>>(Jp, a, -1, -1);
         if (j->h.hi && !j->h.hi_exact && (due & kDueTeaEps)) {
@@ -1080,13 +1109,32 @@ int grid_launch(sopb_job* j, cudaStream_t st, bool updaters, int steps, int due 
         }
     }
     const int fb = (int)std::min<int64_t>((j->n + (kGridBlock / kGridLpb) - 1) / (kGridBlock / kGridLpb), (int64_t)c->sm_count * 8);
+    const bool ext = j->h.discrete || j->h.plane;
+    auto forces = [&](bool prepare) {
+        if (prepare) {
+            if (ext) k_g_forces<true, true><<<fb, kGridBlock, 0, st>>>(Jp, a);
+            else k_g_forces<false, true><<<fb, kGridBlock, 0, st>>>(Jp, a);
+        } else {
+            if (ext) k_g_forces<true, false><<<fb, kGridBlock, 0, st>>>(Jp, a);
+            else k_g_forces<false, false><<<fb, kGridBlock, 0, st>>>(Jp, a);
+        }
+    };
+    // a job without hydrodynamics moves between its two coordinate buffers
+    float4 *xin = j->h.x, *xout = a.F;
+    const bool wide = j->n <= kWideStepBeads;
+    const int sb = (job_pairs(j->n) + step_pairs(wide) - 1) / step_pairs(wide);
     for (int s = 0; s < steps; ++s) {
-        if (j->h.discrete || j->h.plane) k_g_forces<true><<<fb, kGridBlock, 0, st>>>(Jp, a);
-        else k_g_forces<false><<<fb, kGridBlock, 0, st>>>(Jp, a);
         if (!j->h.hi) {
-            k_g_langevin<<<nb, kGridBlock, 0, st>>>(Jp, a);
+            if (ext) {
+                if (wide) k_g_step<true, true><<<sb, kGridBlock, 0, st>>>(Jp, a, xin, xout);
+                else k_g_step<true, false><<<sb, kGridBlock, 0, st>>>(Jp, a, xin, xout);
+            } else {
+                if (wide) k_g_step<false, true><<<sb, kGridBlock, 0, st>>>(Jp, a, xin, xout);
+                else k_g_step<false, false><<<sb, kGridBlock, 0, st>>>(Jp, a, xin, xout);
+            }
+            std::swap(xin, xout);
         } else if (!j->h.hi_exact) {
-            k_hi_prepare<<<nb, kGridBlock, 0, st>>>(Jp, a);
+            forces(true);
             const dim3 tg((j->n + kHiTile - 1) / kHiTile, j->jsplit);
             k_tea_force_partial<<<tg, kHiTile, 0, st>>>(Jp, a, j->jsplit);
             k_tea_integrate<<<nb, kGridBlock, 0, st>>>(Jp, a, j->jsplit);
@@ -1094,7 +1142,7 @@ int grid_launch(sopb_job* j, cudaStream_t st, bool updaters, int steps, int due 
             // the factor is refreshed every step (hi_refresh 1, the
             // reference) or at the updater boundaries due for it
             const bool refresh = j->h.hi_refresh <= 1 || (s == 0 && refresh_first);
-            if (j->n > 128 || j->h.hi_bmode == SOPB_HI_B_REFCOMPAT) k_hi_prepare<<<nb, kGridBlock, 0, st>>>(Jp, a);
+            forces(j->n > 128 || j->h.hi_bmode == SOPB_HI_B_REFCOMPAT);   // k_hi_small prepares for itself
             if (j->n <= 128 && j->h.hi_bmode == SOPB_HI_B_REFCOMPAT) {
                 k_chol_D<<<nb, kGridBlock, 0, st>>>(Jp, a, refresh ? 1 : 0);
                 if (refresh) k_chol_factor_small<<<1, 384, 0, st>>>(Jp, a);
@@ -1116,6 +1164,8 @@ int grid_launch(sopb_job* j, cudaStream_t st, bool updaters, int steps, int due 
             }
         }
     }
+    // an odd number of steps ended in the other buffer
+    if (xin != j->h.x) k_g_copy_back<<<nb, kGridBlock, 0, st>>>(Jp, xin);
     k_g_advance<<<1, 32, 0, st>>>(Jp, steps);
     CUDA_TRY(cudaGetLastError());
     return SOPB_OK;
@@ -1249,7 +1299,7 @@ extern "C" int sopb_job_footprint(const sopb_job_desc* d, size_t* bytes) {
         b += align256(np * 8) + align256(np * row_cap(n, cap_pl, 2) * 2);
         b += align256(np * row_cap(n, cap_pl, 4) * 2) + align256(np * 4) + align256(n * 16);
     }
-    if (grid) b += align256(n * cap_pl * 4);        // Verlet rows
+    if (grid && p.hi_on) b += align256(n * cap_pl * 4);   // Verlet rows (else part of the grid buffers)
     b += n * (16 + 16 + 16 + 4 + 16 + 1);           // bead pools
     if ((p.pulling && p.deltax != 0.0f) || p.indentation || p.pullingPlane)
         b += align256((size_t)(p.log_rows > 0 ? p.log_rows : 1024) * 64);                        // event log
@@ -1513,7 +1563,7 @@ extern "C" int sopb_job_create(sopb_context* c, const sopb_job_desc* d, sopb_job
     const size_t o_vh = o_plcnt + (h.mask ? 0 : align256((size_t)n * 4));
     const size_t o_ppj = o_vh + (h.mask ? align256((size_t)np * 8) : 0);
     const size_t o_plj = o_ppj + (h.mask ? 0 : align256((size_t)n * h.cap_pp * 4));
-    const size_t o_vr = o_plj + (h.mask ? 0 : align256((size_t)n * h.cap_pl * 4));
+    const size_t o_vr = o_plj + (h.hi ? align256((size_t)n * h.cap_pl * 4) : 0);
     const size_t o_nrj = o_vr + (h.mask ? align256((size_t)np * h.cap_u * 2) : 0);
     const size_t o_nrc = o_nrj + (h.mask ? align256((size_t)np * h.cap_nr * 2) : 0);
     const size_t o_xref = o_nrc + (h.mask ? align256((size_t)np * 4) : 0);
@@ -1549,9 +1599,9 @@ extern "C" int sopb_job_create(sopb_context* c, const sopb_job_desc* d, sopb_job
     h.ex_mask = h.grid ? nullptr : (uint32_t*)(base + o_ex);
     h.pp_mask = h.mask ? (uint32_t*)(base + o_ppm) : nullptr;
     h.pp_cnt = h.mask ? nullptr : (int32_t*)(base + o_ppcnt);
-    h.pl_cnt = h.mask ? nullptr : (int32_t*)(base + o_plcnt);
+    h.pl_cnt = h.hi ? (int32_t*)(base + o_plcnt) : nullptr;
     h.pp_j = h.mask ? nullptr : (int32_t*)(base + o_ppj);
-    h.pl_j = h.mask ? nullptr : (int32_t*)(base + o_plj);
+    h.pl_j = h.hi ? (int32_t*)(base + o_plj) : nullptr;
     h.vh = h.mask ? (uint2*)(base + o_vh) : nullptr;
     h.vr = h.mask ? (uint16_t*)(base + o_vr) : nullptr;
     h.nr_j = h.mask ? (uint16_t*)(base + o_nrj) : nullptr;
@@ -1612,6 +1662,18 @@ extern "C" int sopb_job_create(sopb_context* c, const sopb_job_desc* d, sopb_job
             c->beads.release(b0, n);
             delete j;
             return rc2;
+        }
+        if (!h.hi) {
+            GridAux& a = j->aux;
+            h.gvh = a.vh;
+            h.gvr = a.vr;
+            h.cap_u = a.cap_u;
+            h.tile = a.tile;
+            a.cut2 = h.cut2; a.c8 = h.c8; a.ks = h.ks; a.R2 = h.R2;
+            a.hOverZeta = h.hOverZeta; a.tempNorm = h.tempNorm;
+            a.minimization = h.minimization; a.pulling = h.pulling; a.indent = h.indent;
+            a.cov_off = h.cov_off; a.cov_j = h.cov_j; a.cov_r0 = h.cov_r0;
+            a.nat_off = h.nat_off; a.nat_j = h.nat_j; a.nat_par = h.nat_par;
         }
     }
     c->generation++;
@@ -2064,24 +2126,40 @@ extern "C" int sopb_job_pairlist(sopb_job* j, int32_t possible, int32_t* counts,
         }
         return SOPB_OK;
     }
-    if (j->h.mask) {
-        // a resident job's rows are kept per pair of beads: both beads'
-        // partners, then each bead's own, merged in increasing j
-        const int32_t np = job_pairs(n), cap_u = j->h.cap_u;
-        std::vector<uint2> vh(np);
-        std::vector<uint16_t> vr((size_t)np * cap_u);
-        CUDA_TRY(cudaMemcpyAsync(vh.data(), j->h.vh, vh.size() * sizeof(uint2), cudaMemcpyDeviceToHost, c->io));
-        CUDA_TRY(cudaMemcpyAsync(vr.data(), j->h.vr, vr.size() * 2, cudaMemcpyDeviceToHost, c->io));
-        SOPB_TRY(io_end(j, false));
+    if (!possible && (j->h.mask || j->h.gvr)) {
+        // rows kept per pair of beads: both beads' partners, then each bead's
+        // own, merged in increasing j
+        const int32_t np = job_pairs(n), cap_u = j->h.cap_u, tile = j->h.mask ? 1 : j->h.tile;
+        const size_t slots = (size_t)(np + tile - 1) / tile * tile;
+        std::vector<int32_t> heads(4 * (size_t)np), rows_u(slots * cap_u);
+        if (j->h.mask) {
+            std::vector<uint2> vh(np);
+            std::vector<uint16_t> vr((size_t)np * cap_u);
+            CUDA_TRY(cudaMemcpyAsync(vh.data(), j->h.vh, vh.size() * sizeof(uint2), cudaMemcpyDeviceToHost, c->io));
+            CUDA_TRY(cudaMemcpyAsync(vr.data(), j->h.vr, vr.size() * 2, cudaMemcpyDeviceToHost, c->io));
+            SOPB_TRY(io_end(j, false));
+            for (int32_t p = 0; p < np; ++p) {
+                heads[4 * (size_t)p] = vh[p].y & 0xffff;
+                heads[4 * (size_t)p + 1] = vh[p].y >> 16;
+                heads[4 * (size_t)p + 2] = vh[p].x >> 20;
+                heads[4 * (size_t)p + 3] = 0;
+            }
+            std::copy(vr.begin(), vr.end(), rows_u.begin());
+        } else {
+            CUDA_TRY(cudaMemcpyAsync(heads.data(), j->h.gvh, heads.size() * 4, cudaMemcpyDeviceToHost, c->io));
+            CUDA_TRY(cudaMemcpyAsync(rows_u.data(), j->h.gvr, rows_u.size() * 4, cudaMemcpyDeviceToHost, c->io));
+            SOPB_TRY(io_end(j, false));
+        }
         std::vector<int32_t> row;
         for (int32_t i = 0; i < n; ++i) {
-            const int nf = vh[i >> 1].y & 0xffff, n0 = vh[i >> 1].y >> 16, n1 = vh[i >> 1].x >> 20;
-            const uint16_t* r = vr.data() + (size_t)(i >> 1) * cap_u;
-            const uint16_t* own = r + nf + ((i & 1) ? n0 : 0);
-            row.resize((size_t)nf + ((i & 1) ? n1 : n0));
-            std::merge(r, r + nf, own, own + ((i & 1) ? n1 : n0), row.begin());
-            counts[i] = (int32_t)row.size();
-            for (int32_t k = 0; k < cap; ++k) rows[(size_t)i * cap + k] = k < (int32_t)row.size() ? row[k] >> 4 : -1;
+            const int32_t* hd = heads.data() + 4 * (size_t)(i >> 1);
+            const int32_t* r = rows_u.data() + (size_t)((i >> 1) / tile) * tile * cap_u + hd[3];
+            const int32_t* own = r + hd[0] + ((i & 1) ? hd[1] : 0);
+            row.assign(r, r + hd[0]);
+            row.insert(row.end(), own, own + ((i & 1) ? hd[2] : hd[1]));
+            std::sort(row.begin(), row.end());
+            counts[i] = (int32_t)std::min<size_t>(row.size(), (size_t)j->h.cap_pl);
+            for (int32_t k = 0; k < cap; ++k) rows[(size_t)i * cap + k] = k < counts[i] ? row[k] >> 4 : -1;
         }
         return SOPB_OK;
     }
@@ -2109,7 +2187,8 @@ extern "C" int sopb_job_rebuild_lists(sopb_job* j, int32_t possible, int32_t ver
         if (rc) return rc;
         if (verlet) {
             const int wb = (int)std::min<int64_t>((j->n + 7) / 8, (int64_t)c->sm_count * 16);
-            k_g_verlet<<<wb, kGridBlock, 0, c->io>>>(Jp, j->aux, 1);
+            if (j->h.hi) k_g_verlet<<<wb, kGridBlock, 0, c->io>>>(Jp, j->aux, 1);
+            else k_g_pair_rows<<<pair_row_blocks(j), 32 * kPairWarps, 0, c->io>>>(Jp, j->aux, 1);
         }
         if (j->aux.cap_nr && (possible || verlet))
             k_g_near_commit<<<1, 32, 0, c->io>>>(Jp, j->aux, possible ? 1 : 0, verlet ? 1 : 0);

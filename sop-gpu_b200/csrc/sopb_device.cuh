@@ -72,7 +72,9 @@ struct JobDev {
     float2* nat_par;      // (r0^2, -12 eh / r0^2)  (native.cu:112-146)
     int32_t* pp_cnt;      // [n]
     int32_t* pp_j;        // [n * cap_pp]
-    int32_t* pl_cnt;      // [n] Verlet rows of a grid job
+    int4* gvh;            // [ceil(n/2)] Verlet row headers of a grid job without hydrodynamics
+    int32_t* gvr;         // its rows: 16 j (GridAux::vr)
+    int32_t* pl_cnt;      // [n] Verlet rows of a job with hydrodynamics
     int32_t* pl_j;        // [n * cap_pl]
     uint32_t* ex_mask;    // [n * W] bonded + native partners and self
     uint32_t* pp_mask;    // [n * W] possible pairs (MASK mode)
@@ -81,7 +83,8 @@ struct JobDev {
     uint16_t* nr_j;       // [ceil(n/2) * cap_nr] near rows: possible pairs within pairlist_cutoff + skin
     int32_t* nr_cnt;      // [ceil(n/2)]
     float4* x_ref;        // coordinates the near list was built at
-    int32_t cap_u;        // row capacity of vr
+    int32_t cap_u;        // row capacity of vr or gvr
+    int32_t tile;         // pairs per tile of gvr
     int32_t cap_nr;       // near-list row capacity
     int32_t nr_valid;     // 1: the near list holds every pair the next Verlet list can have
     float nr_t;           // r^2 threshold of the near list

@@ -2,18 +2,20 @@
 // CTA (n > ~4096 beads, e.g. a 198k-bead capsid shell) and for jobs with
 // hydrodynamic interactions, whose O(N^2) sums need the whole GPU.
 //
-// One step is a forces kernel followed by the integrator kernel(s).  Every
-// `stride` steps the updater kernels run first; each reads the job's step
-// counter on the device and returns at once when its frequency does not
-// divide it, so a whole stride chunk is one fixed launch sequence that the
-// host captures once in a CUDA graph and replays.  The step counter moves by
-// `stride` in the chunk's last launch.
+// One step of a job without hydrodynamics is one kernel (potentials, noise and
+// move, from one coordinate buffer into the other); with them, a forces kernel
+// followed by the integrator's.  Every `stride` steps the updater kernels run
+// first; each reads the job's step counter on the device and returns at once
+// when its frequency does not divide it, so a whole stride chunk is one fixed
+// launch sequence that the host captures once in a CUDA graph and replays.  The
+// step counter moves by `stride` in the chunk's last launch.
 //
-// Lists are index rows in global memory.  Possible pairs of large jobs come
-// from a cell list (cells no smaller than pairs_threshold, 27-cell search,
-// exact distance test) and each row is then sorted, so the rows equal the
-// reference's brute-force rows (src/Updaters/possiblepairlist_kernel.cu:18-71)
-// entry for entry.
+// Lists are index rows in global memory.  Verlet rows are per bead for jobs
+// with hydrodynamics, per pair of beads without; possible pairs are per bead,
+// for large jobs from a cell list (cells no smaller than pairs_threshold,
+// 27-cell search, exact distance test) whose rows are then sorted, so that
+// they equal the reference's brute-force rows
+// (src/Updaters/possiblepairlist_kernel.cu:18-71) entry for entry.
 #pragma once
 
 #include "sopb_resident.cuh"
@@ -26,8 +28,9 @@ constexpr int kCellMax = 1 << 22;
 constexpr int kSortCap = 2048;   // rows up to this length are sorted in registers
 
 struct GridAux {
+    int32_t n;           // beads
     // per-bead buffers of the grid path
-    float4* F;           // potential forces of the current step
+    float4* F;           // potential forces of the current step (HI), or the second coordinate buffer
     // hydrodynamics (TEA / Cholesky)
     float4* rf;          // rho * g (random force)
     float4* mf;          // molecular force (+ pulling), then D F for Cholesky
@@ -59,7 +62,21 @@ struct GridAux {
     float4* x_ref;       // coordinates it was built at
     int32_t* near;       // [3] drift bits, overflow, usable
     int32_t cap_nr;
+    // Verlet rows per pair of beads of a job without hydrodynamics (whose near
+    // rows are per pair as well: nr_j and nr_cnt by pair)
+    int4* vh;            // [ceil(n/2)] partners of both beads, of the first alone, of the second alone; start
+    int32_t* vr;         // [tiles * tile * cap_u] the three sections of each row: 16 j.  The rows of a tile of
+                         //   pairs lie one after another, each from its start on (tile 1: start 0)
+    int32_t* vtot;       // [tiles] entries of a tile's rows
+    int32_t cap_u, tile;
+    // constants of a step
+    float cut2, c8, ks, R2, hOverZeta, tempNorm;
+    int32_t minimization, pulling, indent;
+    const int32_t *cov_off, *cov_j, *nat_off, *nat_j;
+    const float* cov_r0;
+    const float2* nat_par;
 };
+
 
 __device__ __forceinline__ int64_t job_step(const JobDev* Jp) { return *(volatile const int64_t*)&Jp->step; }
 
@@ -93,11 +110,52 @@ __device__ __forceinline__ void pair_row_v4(const JobDev& J, const float4* __res
     }
 }
 
-// All potentials of every bead at the current coordinates into aux.F; the
-// tip's share accumulates per bead (indentation_kernel.cu:71-128).
+// integrateTea_prepare (bdhitea_kernel.cu:33-65): the random force rho g, the
+// molecular force with pulling applied and a copy of the coordinates.
+__device__ __forceinline__ void hi_prepare(const JobDev& J, const GridAux& aux, int i, float4 xi, float3 f) {
+    uint4 st = J.seeds[i];
+    float4 g = gaussian4(st);
+    J.seeds[i] = st;
+    g.x *= J.var;
+    g.y *= J.var;
+    g.z *= J.var;
+    aux.rf[i] = g;
+    if (J.pulling) {
+        const uint8_t fl = J.flags[i];
+        if (fl == FLAG_FIXED) f.x = f.y = f.z = 0.f;
+        if (fl == FLAG_PULLED) { f.x += J.pullF[0]; f.y += J.pullF[1]; f.z += J.pullF[2]; }
+    }
+    aux.mf[i] = make_float4(f.x, f.y, f.z, 0.f);
+    aux.xc[i] = xi;
+}
+
+// The tip's and the plane's terms of bead i (and the tip's share accumulated
+// per bead, indentation_kernel.cu:71-128).
+template <bool EXT>
+__device__ __forceinline__ void external_terms(const JobDev& J, int i, float4 xi, float3& f) {
+    if (J.indent) {
+        // read from the shared copy here, not held in registers over the pair loop
+        IndentGeom ig;
+        for (int c = 0; c < 3; ++c) { ig.tip[c] = J.tip[c]; ig.micaR[c] = J.micaR[c]; ig.micaN[c] = J.micaN[c]; }
+        ig.tipR = J.tipR; ig.tipAp = J.tipAp; ig.tipBp = J.tipBp; ig.surfAp = J.surfAp; ig.surfBp = J.surfBp;
+        float3 tf;
+        if (EXT && J.discrete) tip_term(xi, ig, f, tf);
+        else indentation_term(xi, ig, f, tf);
+        float4 t = J.tipF[i];
+        t.x += tf.x; t.y += tf.y; t.z += tf.z;
+        J.tipF[i] = t;
+    }
+    if (EXT && J.plane) {
+        const int mask = J.plane_mask[i];
+        if (mask) J.plane_f[i] = plane_term(J, J.plane_displ, mask, xi, J.plane_r0[i], f);
+    }
+}
+
+// All potentials of every bead of a job with hydrodynamics at the current
+// coordinates, into aux.F or (PREP) prepared for the O(N^2) sums.
 // EXT: the job has a discrete surface or a pulling plane (a separate
 // instantiation, so the common one keeps its register budget).
-template <bool EXT>
+template <bool EXT, bool PREP>
 __global__ void __launch_bounds__(kGridBlock)
 k_g_forces(JobDev* __restrict__ Jp, GridAux aux) {
     __shared__ JobDev Js;
@@ -121,56 +179,245 @@ k_g_forces(JobDev* __restrict__ Jp, GridAux aux) {
         }
         f = group_reduce(f, lpb);
         if (act && l == 0) {
-            if (J.indent) {
-                // read from the shared copy here, not held in registers over the pair loop
-                IndentGeom ig;
-                for (int c = 0; c < 3; ++c) { ig.tip[c] = J.tip[c]; ig.micaR[c] = J.micaR[c]; ig.micaN[c] = J.micaN[c]; }
-                ig.tipR = J.tipR; ig.tipAp = J.tipAp; ig.tipBp = J.tipBp; ig.surfAp = J.surfAp; ig.surfBp = J.surfBp;
-                float3 tf;
-                if (EXT && J.discrete) tip_term(xi, ig, f, tf);
-                else indentation_term(xi, ig, f, tf);
-                float4 t = J.tipF[i];
-                t.x += tf.x; t.y += tf.y; t.z += tf.z;
-                J.tipF[i] = t;
-            }
-            if (EXT && J.plane) {
-                const int mask = J.plane_mask[i];
-                if (mask) J.plane_f[i] = plane_term(J, J.plane_displ, mask, xi, J.plane_r0[i], f);
-            }
-            aux.F[i] = make_float4(f.x, f.y, f.z, 0.f);
+            external_terms<EXT>(J, i, xi, f);
+            if (PREP) hi_prepare(J, aux, i, xi, f);
+            else aux.F[i] = make_float4(f.x, f.y, f.z, 0.f);
         }
     }
 }
 
-// ---- Langevin integrator (langevin_kernel.cu:17-58) -------------------------
-__global__ void __launch_bounds__(kGridBlock)
-k_g_langevin(JobDev* __restrict__ Jp, GridAux aux) {
-    __shared__ JobDev Js;
-    load_job<kGridBlock>(Js, Jp);
-    __syncthreads();
-    const JobDev& J = Js;
-    if (J.status) return;
-    for (int i = blockIdx.x * kGridBlock + threadIdx.x; i < J.n; i += gridDim.x * kGridBlock) {
-        float4 f4 = aux.F[i];
-        float3 f = make_float3(f4.x, f4.y, f4.z);
-        if (!J.minimization) {
-            uint4 st = J.seeds[i];
-            const float4 gg = gaussian4(st);
-            J.seeds[i] = st;
-            f.x += gg.x * J.var;
-            f.y += gg.y * J.var;
-            f.z += gg.z * J.var;
-        }
-        if (J.pulling) {
-            const uint8_t fl = J.flags[i];
-            if (fl == FLAG_FIXED) f = make_float3(0.f, 0.f, 0.f);
-            if (fl == FLAG_PULLED) { f.x += J.pullF[0]; f.y += J.pullF[1]; f.z += J.pullF[2]; }
-        }
-        const float4 xi = J.x[i];
-        const float dx = J.hOverZeta * f.x, dy = J.hOverZeta * f.y, dz = J.hOverZeta * f.z;
-        J.x[i] = make_float4(xi.x + dx, xi.y + dy, xi.z + dz, xi.w);
-        J.T[i] += J.tempNorm * (dx * dx + dy * dy + dz * dz);
+// ---- one step without hydrodynamics -----------------------------------------
+// All potentials and the Langevin move (langevin_kernel.cu:17-58) from `xin`
+// into `xout`.  A lane group per pair of beads, in the resident kernel's order
+// of sums: the partners of both beads by the whole group, each bead's own by
+// its half, with its covalent and native terms; then a thread per bead draws
+// the noise and moves the bead.  One gather serves two beads.
+//
+// Bound by the latency of the chain header -> entries -> coordinates, not by
+// bytes: the gathers hit L1 and L2.  Wide groups (16 lanes a pair) shorten a
+// lane's chain and fetch the entries ahead, before the header is there; narrow
+// groups (8 lanes) do less work per pair, and their CTA's rows, which lie one
+// after another, arrive in shared memory by one bulk copy while the bonded
+// terms are computed.
+//
+// Measured per step (free globules, 20 A lists, rebuilds included): 5011 beads
+// 9.5 us wide, 15.3 narrow; 20000 beads 16.6 and 18.8; 30000 beads 20.8 and
+// 19.0 -- the line lies between.  A clamped chain of 5011 beads takes 10.7 us
+// per step, 14.0 with a lane group per bead and the integrator as a kernel of
+// its own (whose forces and moves took 16.0 + 5.1 us under the profiler, this
+// kernel 12.0); a 198000-bead shell 106 us, 126 before (88 + 6 us, now 70).
+constexpr int kWideStepBeads = 24576;   // up to this size the step takes wide groups
+__host__ __device__ constexpr int step_pairs(bool wide) { return kGridBlock / (wide ? 16 : 8); }   // pairs per CTA
+constexpr int kStepRow = 192;           // row entries per pair that a CTA has shared memory for
+constexpr uint32_t kStepWaitLimit = 1u << 20;
+
+// Entries [k0 + l, k1) of a row in steps of G, four gathers in flight:
+// term(u, coordinates) for the u-th of four.
+template <typename Term>
+__device__ __forceinline__ void gather4(const int32_t* row, int k, int k1, int G, const char* xb, Term term) {
+    for (; k + 3 * G < k1; k += 4 * G) {
+        float4 q[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) q[u] = bead_at(xb, row[k + u * G]);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) term(u, q[u]);
     }
+    float4 q[3];
+#pragma unroll
+    for (int u = 0; u < 3; ++u)
+        if (k + u * G < k1) q[u] = bead_at(xb, row[k + u * G]);
+#pragma unroll
+    for (int u = 0; u < 3; ++u)
+        if (k + u * G < k1) term(u, q[u]);
+}
+
+template <bool EXT, bool WIDE>
+__global__ void __launch_bounds__(kGridBlock, WIDE ? 3 : 4)
+k_g_step(JobDev* __restrict__ Jp, const GridAux aux, const float4* __restrict__ xin, float4* __restrict__ xout) {
+    constexpr int G = WIDE ? 16 : 8, kPairs = step_pairs(WIDE);
+    __shared__ float4 Fs[2 * kPairs];
+    __shared__ __align__(128) int32_t rows_s[WIDE ? 4 : kPairs * kStepRow];
+    __shared__ __align__(8) uint64_t bar_s;
+    __shared__ int in_smem;
+    const int tid = threadIdx.x, n = aux.n;
+    const int p0 = blockIdx.x * kPairs, p = p0 + tid / G;
+    const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&bar_s);
+    const int32_t* rows_g = aux.vr + (size_t)(WIDE ? p : p0) * aux.cap_u;
+    // the CTA's rows into shared memory with one bulk copy, if they fit
+    if (!WIDE && tid == 0) {
+        const int total = aux.vtot[blockIdx.x];
+        in_smem = total <= kPairs * kStepRow;
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        const uint32_t bytes = in_smem ? 4u * (uint32_t)total : 0u;
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+        if (bytes)
+            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                             (uint32_t)__cvta_generic_to_shared(rows_s)),
+                         "l"(rows_g), "r"(bytes), "r"(bar)
+                         : "memory");
+    }
+    const PairGroup<WIDE> g(4, tid & 31, G);
+    const int i = 2 * p + g.h;
+    const bool act = i < n;
+    const char* xb = reinterpret_cast<const char*>(xin);
+    const int own = g.own_lanes();
+    // meanwhile the row's header, the two beads and the bead's maps
+    const int status = Jp->status;
+    int4 hd = make_int4(0, 0, 0, 0);
+    float4 x0 = make_float4(1.0e18f, 1.0e18f, 1.0e18f, 0.f), x1 = x0;
+    int c0 = 0, c1 = 0, n0 = 0, n1 = 0;
+    int pre[WIDE ? 4 : 1];
+    if (WIDE)                              // readable whatever the row's length
+#pragma unroll
+        for (int u = 0; u < 4; ++u) pre[u] = 2 * p < n ? rows_g[min(g.l + u * G, aux.cap_u - 1)] : 0;
+    if (2 * p < n) {
+        hd = aux.vh[p];
+        x0 = xin[2 * p];
+        if (2 * p + 1 < n) x1 = xin[2 * p + 1];
+    }
+    if (act && g.owns()) {
+        c0 = aux.cov_off[i] + g.lh;
+        c1 = aux.cov_off[i + 1];
+        n0 = aux.nat_off[i] + g.lh;
+        n1 = aux.nat_off[i + 1];
+    }
+    const float4 xi = g.h ? x1 : x0;
+    const int k_own = hd.x + (g.h ? hd.y : 0) + g.lh, e_own = hd.x + hd.y + (g.h ? hd.z : 0);
+    int w[WIDE ? 4 : 1];
+    if (WIDE)
+#pragma unroll
+        for (int u = 0; u < 4; ++u) w[u] = g.owns() && k_own + u * own < e_own ? rows_g[k_own + u * own] : -1;
+    // the first bond and the first two contacts of the lane
+    int cj = 0, nj0 = 0, nj1 = 0;
+    float cr = 0.f;
+    float2 np0 = make_float2(0.f, 0.f), np1 = np0;
+    if (c0 < c1) {
+        cj = aux.cov_j[c0];
+        cr = aux.cov_r0[c0];
+    }
+    if (n0 < n1) {
+        nj0 = aux.nat_j[n0];
+        np0 = aux.nat_par[n0];
+    }
+    if (n0 + own < n1) {
+        nj1 = aux.nat_j[n0 + own];
+        np1 = aux.nat_par[n0 + own];
+    }
+    float3 fb = make_float3(0.f, 0.f, 0.f);
+    auto bonded = [&] {
+        const float4 qc = xin[cj], q0 = xin[nj0], q1 = xin[nj1];
+        if (c0 < c1) fene_term(xi, qc, cr, aux.ks, aux.R2, fb);
+        if (n0 < n1) native_term(xi, q0, np0, fb);
+        if (n0 + own < n1) native_term(xi, q1, np1, fb);
+        for (int k = c0 + own; k < c1; k += own) fene_term(xi, xin[aux.cov_j[k]], aux.cov_r0[k], aux.ks, aux.R2, fb);
+        for (int k = n0 + 2 * own; k < n1; k += own) native_term(xi, xin[aux.nat_j[k]], aux.nat_par[k], fb);
+    };
+    if (!WIDE) bonded();                   // they do not need the rows
+    if (EXT && act && g.owns() && Jp->discrete) mica_partial(*Jp, i, xi, g.lh, own, fb);
+    if (!WIDE) {
+        __syncthreads();                       // the barrier is set up
+        bool there = false;
+        for (uint32_t it = 0; it < kStepWaitLimit && !there; ++it) {
+            uint32_t ok;
+            asm volatile(
+                "{\n\t.reg .pred P1;\n\t"
+                "mbarrier.try_wait.parity.shared::cta.b64 P1, [%1], 0;\n\t"
+                "selp.b32 %0, 1, 0, P1;\n\t}\n"
+                : "=r"(ok)
+                : "r"(bar)
+                : "memory");
+            there = ok;
+        }
+        if (!__syncthreads_and(there)) {       // the copy did not arrive
+            if (tid == 0) atomicMax(&Jp->status, SOPB_ERR_TIMEOUT);
+            return;
+        }
+    }
+    if (status) return;
+    const float cut2 = aux.cut2;
+    const float3 zero = make_float3(0.f, 0.f, 0.f);
+    float3 a0 = zero, a1 = zero, b0 = zero, b1 = zero, f = zero;
+    auto both = [&](int u, float4 q) {
+        pair_term8(x0, q, cut2, WIDE || u % 2 == 0 ? a0 : b0);
+        pair_term8(x1, q, cut2, WIDE || u % 2 == 0 ? a1 : b1);
+    };
+    auto single = [&](int, float4 q) { pair_term8(xi, q, cut2, f); };
+    if (WIDE) {
+        // four entries of the lane at a time, the next ones fetched before
+        // these ones' gathers are used
+        for (int k = g.l; k < hd.x; k += 4 * G) {
+            int o[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) o[u] = k + u * G < hd.x ? pre[u] : -1;
+            if (k + 4 * G < hd.x) {
+#pragma unroll
+                for (int u = 0; u < 4; ++u) pre[u] = rows_g[min(k + (4 + u) * G, aux.cap_u - 1)];
+            }
+            float4 q[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (o[u] >= 0) q[u] = bead_at(xb, o[u]);
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (o[u] >= 0) both(u, q[u]);
+        }
+        float4 q[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (w[u] >= 0) q[u] = bead_at(xb, w[u]);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (w[u] >= 0) single(u, q[u]);
+        if (g.owns()) gather4(rows_g, k_own + 4 * own, e_own, own, xb, single);
+        bonded();
+    } else {
+        auto sums = [&](const int32_t* row) {
+            gather4(row, g.l, hd.x, G, xb, both);
+            gather4(row, k_own, e_own, own, xb, single);
+        };
+        if (in_smem) sums(rows_s + hd.w);
+        else sums(rows_g + hd.w);
+    }
+    const float3 fs = pair_sum(g, a0, a1, b0, b1);
+    f = make_float3(fmaf(aux.c8, f.x, fb.x), fmaf(aux.c8, f.y, fb.y), fmaf(aux.c8, f.z, fb.z));
+    f = pair_total(fs, f, aux.c8, g);
+    if (g.lh == 0 && act) {
+        if (EXT || aux.indent) external_terms<EXT>(*Jp, i, xi, f);
+        Fs[i - 2 * p0] = make_float4(f.x, f.y, f.z, 0.f);
+    }
+    __syncthreads();
+    const int b = 2 * p0 + tid;
+    if (tid < 2 * kPairs && b < n) {
+        f = make_float3(Fs[tid].x, Fs[tid].y, Fs[tid].z);
+        if (!aux.minimization) {
+            uint4 st = Jp->seeds[b];
+            const float var = Jp->var;
+            const float4 gg = gaussian4(st);
+            Jp->seeds[b] = st;
+            f.x += gg.x * var;
+            f.y += gg.y * var;
+            f.z += gg.z * var;
+        }
+        if (aux.pulling) {
+            const uint8_t fl = Jp->flags[b];
+            if (fl == FLAG_FIXED) f = make_float3(0.f, 0.f, 0.f);
+            if (fl == FLAG_PULLED) { f.x += Jp->pullF[0]; f.y += Jp->pullF[1]; f.z += Jp->pullF[2]; }
+        }
+        const float4 xi0 = xin[b];
+        const float dx = aux.hOverZeta * f.x, dy = aux.hOverZeta * f.y, dz = aux.hOverZeta * f.z;
+        xout[b] = make_float4(xi0.x + dx, xi0.y + dy, xi0.z + dz, xi0.w);
+        Jp->T[b] += aux.tempNorm * (dx * dx + dy * dy + dz * dz);
+    }
+}
+
+// The coordinates after an odd number of steps, back into the job's own buffer
+// (a failed job's steps wrote nothing: it keeps its coordinates).
+__global__ void __launch_bounds__(kGridBlock)
+k_g_copy_back(JobDev* __restrict__ Jp, const float4* __restrict__ x) {
+    const JobDev& J = *Jp;
+    if (J.status) return;
+    for (int i = blockIdx.x * kGridBlock + threadIdx.x; i < J.n; i += gridDim.x * kGridBlock) J.x[i] = x[i];
 }
 
 // ---- updaters ----------------------------------------------------------------
@@ -677,7 +924,8 @@ __device__ __forceinline__ int append_hits(int32_t* row, int cap, int& cnt, unsi
     return over;
 }
 
-// Verlet rows (pairlist_kernel.cu:33-76), order kept: a warp per bead, each
+// Verlet rows (pairlist_kernel.cu:33-76) of a job with hydrodynamics, per
+// bead, order kept: a warp per bead, each
 // lane testing four consecutive candidates of the warp's 128 (four gathers in
 // flight), an order-preserving warp scan placing the hits.  From the near
 // rows when they are usable and no bead drifted too far; else from the
@@ -734,6 +982,239 @@ k_g_verlet(JobDev* __restrict__ Jp, GridAux a, int force) {
                 a.x_ref[i] = xi;
             }
         }
+    }
+    if (err) atomicMax(&Jp->status, err);
+    if (over) atomicOr(&a.near[1], 1);
+}
+
+// Whether a sorted row of cnt entries holds v.
+__device__ __forceinline__ bool in_sorted(const int32_t* row, int cnt, int v) {
+    int lo = 0, hi = cnt;
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (row[mid] < v) lo = mid + 1;
+        else hi = mid;
+    }
+    return lo < cnt && row[lo] == v;
+}
+
+// Verlet rows (pairlist_kernel.cu:33-76) of a job without hydrodynamics, per
+// pair of beads (2p, 2p + 1): the partners of both, of the first alone, of the
+// second alone.  A warp per pair.
+// Candidates are 8 q with bit 0 when the first bead may pair with q and bit 1
+// when the second may, in this order: the first bead's possible partners
+// (increasing j; a search in the second bead's row gives bit 1), then those of
+// the second bead that are not the first one's.  The near rows hold the
+// candidates within pairlist_cutoff + skin of a bead they may pair with, in
+// the same order, so a rebuild from them places the same hits in the same
+// order as one from all candidates.
+// As in the resident kernel, ballots give each hit its place in its section
+// (kept in a register for the first eight rounds of 32), then the hits are
+// stored.  More than max_pairs partners of a bead sets err.
+// A CTA takes a tile of pairs at a time and gives their rows consecutive places
+// (any order: a header holds its row's start), four rounds' gathers in flight.
+// Bound by latency: 206 us for the near rows of a 198000-bead shell (195
+// with a row per bead, which the step then gathers twice), 250 with one round's
+// gathers in flight.  A renewal of the near rows takes 1.6 ms
+// (0.56), mostly the searches; it is one of thousands of rebuilds.
+constexpr int kPairWarps = 4;      // warps per CTA
+constexpr int kPairBuf = 1024;     // entries of a possible row kept in shared memory for the searches
+constexpr int kPairTmp = 448;      // entries of a row that are near, before the searches
+__device__ __forceinline__ int pair_hit(const float4* __restrict__ x, float4 x0, float4 x1, float t, int e) {
+    const float4 q = x[e >> 3];
+    return ((dist2_rn(x0, q) < t ? 1 : 0) | (dist2_rn(x1, q) < t ? 2 : 0)) & e;
+}
+template <typename Cand>
+__device__ __forceinline__ void build_pair_row(const JobDev& J, const GridAux& a, int p, float4 x0, float4 x1, int rounds,
+                                               Cand cand, int* alloc, int& err) {
+    const int l = threadIdx.x & 31, cap = a.cap_u & ~3;
+    const unsigned below = (1u << l) - 1u, all = 0xffffffffu;
+    int cf = 0, c0 = 0, c1 = 0;
+    auto take = [&](int hit) {
+        const unsigned mf = __ballot_sync(all, hit == 3), m0 = __ballot_sync(all, hit == 1), m1 = __ballot_sync(all, hit == 2);
+        const int at = (hit == 3 ? cf : (hit == 1 ? c0 : c1)) + __popc((hit == 3 ? mf : (hit == 1 ? m0 : m1)) & below);
+        cf += __popc(mf);
+        c0 += __popc(m0);
+        c1 += __popc(m1);
+        return at;
+    };
+    auto round = [&](int e, int& at) {
+        const int hit = pair_hit(J.x, x0, x1, J.pl_t, e);
+        at = take(hit);
+        return (e & ~7) | hit;
+    };
+    int w[kKeptRounds], place[kKeptRounds];
+#pragma unroll
+    for (int u = 0; u < kKeptRounds; ++u) w[u] = u < rounds ? cand(u) : 0;
+#pragma unroll
+    for (int u = 0; u < kKeptRounds; u += 4)
+        if (u < rounds) {
+            // four rounds' gathers in flight; an entry 0 hits nothing
+            float4 q[4];
+#pragma unroll
+            for (int v = 0; v < 4; ++v) q[v] = J.x[w[u + v] >> 3];
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+                const int hit = ((dist2_rn(x0, q[v]) < J.pl_t ? 1 : 0) | (dist2_rn(x1, q[v]) < J.pl_t ? 2 : 0)) & w[u + v];
+                w[u + v] = (w[u + v] & ~7) | hit;
+                place[u + v] = take(hit);
+            }
+        }
+    const int kf = cf, k0 = c0, k1 = c1;
+    int at;
+    for (int u = kKeptRounds; u < rounds; ++u) round(cand(u), at);
+    int nf = cf, n0 = c0, n1 = c1;
+    if (max(n0, n1) + nf > J.cap_pl) {
+        err = SOPB_STATUS_CAPACITY;
+        nf = min(nf, cap);
+        n0 = min(n0, cap - nf);
+        n1 = min(n1, cap - nf - n0);
+    }
+    const int len = nf + n0 + n1;
+    int start = 0;
+    if (a.tile > 1) {
+        if (l == 0) start = atomicAdd(alloc, (len + 3) & ~3);
+        start = __shfl_sync(all, start, 0);
+    }
+    int32_t* dst = a.vr + (size_t)(p / a.tile) * a.tile * a.cap_u + start;
+    auto store = [&](int v, int pos) {
+        const int hit = v & 3;
+        pos += hit == 3 ? 0 : (hit == 1 ? nf : nf + n0);
+        if (hit && pos < len) dst[pos] = 2 * (v & ~7);       // 16 j
+    };
+#pragma unroll
+    for (int u = 0; u < kKeptRounds; ++u)
+        if (u < rounds) store(w[u], place[u]);
+    cf = kf;
+    c0 = k0;
+    c1 = k1;
+    for (int u = kKeptRounds; u < rounds; ++u) {
+        const int v = round(cand(u), at);
+        store(v, at);
+    }
+    if (l == 0) a.vh[p] = make_int4(nf, n0, n1, start);
+}
+
+// The near row of pair p: its candidates within nr_t of a bead they may pair
+// with.  First the entries of a possible row that are near at all, then the
+// searches in the other row for those.
+__device__ __forceinline__ int build_near_row(const JobDev& J, int32_t* nrow, int cap, const int32_t* s0, int c0, const int32_t* s1,
+                                              int c1, float4 x0, float4 x1, int32_t* tmp) {
+    const int l = threadIdx.x & 31;
+    const unsigned below = (1u << l) - 1u, all = 0xffffffffu;
+    int count = 0;
+    for (int h = 0; h < 2; ++h) {
+        const int32_t* own = h ? s1 : s0;
+        const int32_t* other = h ? s0 : s1;
+        const int cown = h ? c1 : c0, cother = h ? c0 : c1;
+        for (int kb = 0; kb < cown;) {
+            // up to kPairTmp near entries of the row
+            int m = 0;
+            for (; kb < cown && m + 128 <= kPairTmp; kb += 128) {
+                int q[4];
+                float4 xq[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) q[u] = own[min(kb + 32 * u + l, cown - 1)];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) xq[u] = J.x[q[u]];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    unsigned bits = (dist2_rn(x0, xq[u]) < J.nr_t ? 1u : 0u) | (dist2_rn(x1, xq[u]) < J.nr_t ? 2u : 0u);
+                    if (h) bits &= 2u;
+                    if (kb + 32 * u + l >= cown) bits = 0;
+                    const unsigned v = __ballot_sync(all, bits != 0);
+                    if (bits) tmp[m + __popc(v & below)] = 8 * q[u] + (int)bits;
+                    m += __popc(v);
+                }
+            }
+            __syncwarp();
+            for (int k = 0; k < m; k += 32) {
+                int e = k + l < m ? tmp[k + l] : 0;
+                // of the first row: bit 1 stands if the second one holds it
+                // too; of the second row: only what the first one does not hold
+                if (!h && (e & 2) && !in_sorted(other, cother, e >> 3)) e &= ~2;
+                if (h && e && in_sorted(other, cother, e >> 3)) e = 0;
+                const unsigned v = __ballot_sync(all, e & 3);
+                const int pos = count + __popc(v & below);
+                if ((e & 3) && pos < cap) nrow[pos] = e;
+                count += __popc(v);
+            }
+            __syncwarp();
+        }
+    }
+    return count;
+}
+
+__global__ void __launch_bounds__(32 * kPairWarps)
+k_g_pair_rows(JobDev* __restrict__ Jp, GridAux a, int force) {
+    __shared__ JobDev Js;
+    __shared__ int32_t buf[kPairWarps][2][kPairBuf], tmp[kPairWarps][kPairTmp];
+    __shared__ int alloc;
+    load_job<32 * kPairWarps>(Js, Jp);
+    __syncthreads();
+    const JobDev& J = Js;
+    const int64_t step = J.step;
+    if (J.status || (!force && (step % J.stride != 0 || step % J.pairs_freq != 0))) return;
+    const bool near = verlet_from_near(J, a, step, force);
+    const int l = threadIdx.x & 31, wp = threadIdx.x >> 5, np = (J.n + 1) >> 1;
+    const int group = max(a.tile, kPairWarps), groups = (np + group - 1) / group;
+    int err = 0, over = 0;
+    for (int t = blockIdx.x; t < groups; t += gridDim.x) {
+        if (threadIdx.x == 0) alloc = 0;
+        __syncthreads();
+        for (int p = t * group + wp; p < min(np, (t + 1) * group); p += kPairWarps) {
+            const bool two = 2 * p + 1 < J.n;
+            const float4 x0 = J.x[2 * p], x1 = J.x[two ? 2 * p + 1 : 2 * p];
+            int32_t* nrow = a.nr_j ? a.nr_j + (size_t)p * a.cap_nr : nullptr;
+            int count = near ? a.nr_cnt[p] : 0;
+            bool from_near = near;
+            int c0 = 0, c1 = 0;
+            const int32_t *s0 = nullptr, *s1 = nullptr;
+            if (!near) {
+                c0 = J.pp_cnt[2 * p];
+                c1 = two ? J.pp_cnt[2 * p + 1] : 0;
+                const int32_t *r0 = J.pp_j + (size_t)(2 * p) * J.cap_pp, *r1 = r0 + J.cap_pp;
+                s0 = r0;
+                s1 = r1;
+                if (c0 <= kPairBuf) {
+                    for (int k = l; k < c0; k += 32) buf[wp][0][k] = r0[k];
+                    s0 = buf[wp][0];
+                }
+                if (c1 <= kPairBuf) {
+                    for (int k = l; k < c1; k += 32) buf[wp][1][k] = r1[k];
+                    s1 = buf[wp][1];
+                }
+                __syncwarp();
+                if (nrow) {
+                    count = build_near_row(J, nrow, a.cap_nr, s0, c0, s1, c1, x0, x1, tmp[wp]);
+                    if (l == 0) {
+                        a.nr_cnt[p] = min(count, a.cap_nr);
+                        a.x_ref[2 * p] = x0;
+                        if (two) a.x_ref[2 * p + 1] = x1;
+                    }
+                    if (count > a.cap_nr) over = 1;
+                    else from_near = true;
+                    __syncwarp();
+                }
+            }
+            if (from_near) {
+                build_pair_row(J, a, p, x0, x1, (count + 31) >> 5,
+                               [&](int u) { return 32 * u + l < count ? nrow[32 * u + l] : 0; }, &alloc, err);
+            } else {
+                // no near row: straight from the candidates
+                const int rounds0 = (c0 + 31) >> 5;
+                auto cand = [&](int u) {
+                    const int k = 32 * (u < rounds0 ? u : u - rounds0) + l;
+                    if (u < rounds0) return k < c0 ? 8 * s0[k] + 1 + (in_sorted(s1, c1, s0[k]) ? 2 : 0) : 0;
+                    return k < c1 && !in_sorted(s0, c0, s1[k]) ? 8 * s1[k] + 2 : 0;
+                };
+                build_pair_row(J, a, p, x0, x1, rounds0 + ((c1 + 31) >> 5), cand, &alloc, err);
+            }
+            __syncwarp();
+        }
+        __syncthreads();
+        if (threadIdx.x == 0 && a.tile > 1) a.vtot[t] = alloc;
+        __syncthreads();
     }
     if (err) atomicMax(&Jp->status, err);
     if (over) atomicOr(&a.near[1], 1);

@@ -94,34 +94,6 @@ __device__ __forceinline__ bool tea_eps_due(const JobDev& J, int64_t step) {
     return step % J.stride == 0 && step % J.eps_freq == 0;
 }
 
-// integrateTea_prepare (bdhitea_kernel.cu:33-65): random force rho*g,
-// molecular force with pulling applied, coordinate copy.
-__global__ void __launch_bounds__(kGridBlock)
-k_hi_prepare(JobDev* __restrict__ Jp, GridAux aux) {
-    __shared__ JobDev Js;
-    load_job<kGridBlock>(Js, Jp);
-    __syncthreads();
-    const JobDev& J = Js;
-    if (J.status) return;
-    for (int i = blockIdx.x * kGridBlock + threadIdx.x; i < J.n; i += gridDim.x * kGridBlock) {
-        uint4 st = J.seeds[i];
-        float4 g = gaussian4(st);
-        J.seeds[i] = st;
-        g.x *= J.var;
-        g.y *= J.var;
-        g.z *= J.var;
-        aux.rf[i] = g;
-        float4 f = aux.F[i];
-        if (J.pulling) {
-            const uint8_t fl = J.flags[i];
-            if (fl == FLAG_FIXED) f.x = f.y = f.z = 0.f;
-            if (fl == FLAG_PULLED) { f.x += J.pullF[0]; f.y += J.pullF[1]; f.z += J.pullF[2]; }
-        }
-        aux.mf[i] = f;
-        aux.xc[i] = J.x[i];
-    }
-}
-
 // ---- TEA epsilon (updater) --------------------------------------------------
 __global__ void __launch_bounds__(kHiTile)
 k_tea_eps_partial(JobDev* __restrict__ Jp, GridAux aux, int jsplit, int force) {

@@ -240,26 +240,10 @@ __device__ __forceinline__ float3 shfl3_xor(float3 f, int o) {
                        __shfl_xor_sync(0xffffffffu, f.z, o));
 }
 
-// The both-section: S[w] of the lane's bead, unscaled sums of d / r^8.  All
-// lanes of the warp take part (an empty row where a group has no pair).
+// S[w] of the lane's bead from the lanes' both-section sums: a of lane l, b
+// (narrow) of lane l + G.  All lanes of the warp take part.
 template <bool WIDE>
-__device__ __forceinline__ float3 row_both(const uint16_t* __restrict__ row, int cnt, const PairGroup<WIDE>& g,
-                                           const char* xb, float4 x0, float4 x1, float cut2) {
-    float3 a0 = make_float3(0.f, 0.f, 0.f), a1 = a0, b0 = a0, b1 = a0;
-    int k = g.l;
-    for (; k + g.G < cnt; k += 2 * g.G) {
-        const int o0 = row[k], o1 = row[k + g.G];
-        const float4 q0 = bead_at(xb, o0), q1 = bead_at(xb, o1);
-        pair_term8(x0, q0, cut2, a0);
-        pair_term8(x1, q0, cut2, a1);
-        pair_term8(x0, q1, cut2, WIDE ? a0 : b0);
-        pair_term8(x1, q1, cut2, WIDE ? a1 : b1);
-    }
-    if (k < cnt) {
-        const float4 q = bead_at(xb, row[k]);
-        pair_term8(x0, q, cut2, a0);
-        pair_term8(x1, q, cut2, a1);
-    }
+__device__ __forceinline__ float3 pair_sum(const PairGroup<WIDE>& g, float3 a0, float3 a1, float3 b0, float3 b1) {
     __syncwarp();
     float3 s;
     if (WIDE) {
@@ -276,10 +260,33 @@ __device__ __forceinline__ float3 row_both(const uint16_t* __restrict__ row, int
     return s;
 }
 
+// The both-section: unscaled sums of d / r^8 (an empty row where a group has
+// no pair).
+template <bool WIDE, typename Entry>
+__device__ __forceinline__ float3 row_both(const Entry* __restrict__ row, int cnt, const PairGroup<WIDE>& g,
+                                           const char* xb, float4 x0, float4 x1, float cut2) {
+    float3 a0 = make_float3(0.f, 0.f, 0.f), a1 = a0, b0 = a0, b1 = a0;
+    int k = g.l;
+    for (; k + g.G < cnt; k += 2 * g.G) {
+        const int o0 = row[k], o1 = row[k + g.G];
+        const float4 q0 = bead_at(xb, o0), q1 = bead_at(xb, o1);
+        pair_term8(x0, q0, cut2, a0);
+        pair_term8(x1, q0, cut2, a1);
+        pair_term8(x0, q1, cut2, WIDE ? a0 : b0);
+        pair_term8(x1, q1, cut2, WIDE ? a1 : b1);
+    }
+    if (k < cnt) {
+        const float4 q = bead_at(xb, row[k]);
+        pair_term8(x0, q, cut2, a0);
+        pair_term8(x1, q, cut2, a1);
+    }
+    return pair_sum(g, a0, a1, b0, b1);
+}
+
 // A bead's own section, its bonded maps and its surface beads, over the V/4
 // lanes of its half of the group.
-template <bool WIDE>
-__device__ __forceinline__ float3 row_own(const uint16_t* __restrict__ row, int cnt, const PairGroup<WIDE>& g, const char* xb,
+template <bool WIDE, typename Entry>
+__device__ __forceinline__ float3 row_own(const Entry* __restrict__ row, int cnt, const PairGroup<WIDE>& g, const char* xb,
                                           float4 xi, float cut2, float c8) {
     float3 f = make_float3(0.f, 0.f, 0.f);
     const int step = g.own_lanes();
@@ -322,6 +329,12 @@ __device__ __forceinline__ void for_partners(const JobDev& J, int i, Visit visit
         for (int k = 0; k < hd.nf; ++k) visit(row[k] >> 4);
         const uint16_t* own = row + hd.nf + ((i & 1) ? hd.n0 : 0);
         for (int k = 0; k < ((i & 1) ? hd.n1 : hd.n0); ++k) visit(own[k] >> 4);
+    } else if (J.gvr) {
+        const int4 hd = J.gvh[i >> 1];
+        const int32_t* row = J.gvr + (size_t)((i >> 1) / J.tile) * J.tile * J.cap_u + hd.w;
+        for (int k = 0; k < hd.x; ++k) visit(row[k] >> 4);
+        const int32_t* own = row + hd.x + ((i & 1) ? hd.y : 0);
+        for (int k = 0; k < ((i & 1) ? hd.z : hd.y); ++k) visit(own[k] >> 4);
     } else {
         const int32_t* row = J.pl_j + (size_t)i * J.cap_pl;
         for (int k = 0; k < J.pl_cnt[i]; ++k) visit(row[k]);
@@ -1193,26 +1206,43 @@ k_forces_only(const JobDev* __restrict__ jobs, const int32_t* __restrict__ ids, 
     __syncthreads();
     const JobDev& J = Js;
     const int n = J.n, tid = threadIdx.x;
-    // resident jobs: a lane group per pair of beads; others: lpb lanes per bead
+    // rows per pair of beads: a lane group per pair; others: lpb lanes per bead
+    const bool pairs = J.mask || J.gvr;
     const PairGroup<false> pg(J.lpb, tid & 31, 0);
-    const int G = J.mask ? pg.G : J.lpb, ng = blockDim.x / G, tasks = J.mask ? job_pairs(n) : n;
-    const int lh = J.mask ? pg.lh : tid % G, h = J.mask ? pg.h : 0;
+    const int G = pairs ? pg.G : J.lpb, ng = blockDim.x / G, tasks = pairs ? job_pairs(n) : n;
+    const int lh = pairs ? pg.lh : tid % G, h = pairs ? pg.h : 0;
     IndentGeom ig;
     for (int c = 0; c < 3; ++c) { ig.tip[c] = J.tip[c]; ig.micaR[c] = J.micaR[c]; ig.micaN[c] = J.micaN[c]; }
     ig.tipR = J.tipR; ig.tipAp = J.tipAp; ig.tipBp = J.tipBp; ig.surfAp = J.surfAp; ig.surfBp = J.surfBp;
     for (int base = 0; base < tasks; base += ng) {
-        const int t = base + tid / G, i = J.mask ? 2 * t + h : t;
+        const int t = base + tid / G, i = pairs ? 2 * t + h : t;
         const bool act = i < n;
         const float4 xi = J.x[act ? i : 0];
         float3 f = make_float3(0.f, 0.f, 0.f);
-        if (J.mask) {
-            RowHead hd = unpack_head(J.vh[t < tasks ? t : 0]);
-            if (t >= tasks) hd.nf = hd.n0 = hd.n1 = 0;
-            const uint16_t* row = J.vr + (size_t)(t < tasks ? t : 0) * J.cap_u;
-            const float4 x0 = J.x[t < tasks ? 2 * t : 0], x1 = J.x[2 * t + 1 < n ? 2 * t + 1 : 0];
+        if (pairs) {
+            const int p = t < tasks ? t : 0;
+            int nf = 0, n0 = 0, n1 = 0, start = 0;
+            if (t < tasks && J.mask) {
+                const RowHead hd = unpack_head(J.vh[p]);
+                nf = hd.nf;
+                n0 = hd.n0;
+                n1 = hd.n1;
+            } else if (t < tasks) {
+                const int4 hd = J.gvh[p];
+                nf = hd.x;
+                n0 = hd.y;
+                n1 = hd.z;
+                start = hd.w;
+            }
+            const float4 x0 = J.x[2 * p], x1 = J.x[2 * p + 1 < n ? 2 * p + 1 : 2 * p];
             const char* xb = reinterpret_cast<const char*>(J.x);
-            const float3 fs = row_both(row, hd.nf, pg, xb, x0, x1, J.cut2);
-            f = row_own(row + hd.nf + (h ? hd.n0 : 0), h ? hd.n1 : hd.n0, pg, xb, xi, J.cut2, J.c8);
+            float3 fs;
+            auto sums = [&](auto* row) {
+                fs = row_both(row, nf, pg, xb, x0, x1, J.cut2);
+                f = row_own(row + nf + (h ? n0 : 0), h ? n1 : n0, pg, xb, xi, J.cut2, J.c8);
+            };
+            if (J.mask) sums(J.vr + (size_t)p * J.cap_u);
+            else sums(J.gvr + (size_t)(p / J.tile) * J.tile * J.cap_u + start);
             if (act) {
                 bonded_global(J, J.x, i, xi, pg, f);
                 if (J.discrete) mica_partial(J, i, xi, lh, pg.own_lanes(), f);
