@@ -1108,7 +1108,7 @@ int grid_launch(sopb_job* j, cudaStream_t st, bool updaters, int steps, int due 
             k_tea_beta<<<1, 256, 0, st>>>(Jp, a, 0);
         }
     }
-    const int fb = (int)std::min<int64_t>((j->n + (kGridBlock / kGridLpb) - 1) / (kGridBlock / kGridLpb), (int64_t)c->sm_count * 8);
+    const int fb = (int)std::min<int64_t>((j->n + (kGridBlock / kForceLpb) - 1) / (kGridBlock / kForceLpb), (int64_t)c->sm_count * 8);
     const bool ext = j->h.discrete || j->h.plane;
     auto forces = [&](bool prepare) {
         if (prepare) {
@@ -1135,9 +1135,10 @@ int grid_launch(sopb_job* j, cudaStream_t st, bool updaters, int steps, int due 
             std::swap(xin, xout);
         } else if (!j->h.hi_exact) {
             forces(true);
-            const dim3 tg((j->n + kHiTile - 1) / kHiTile, j->jsplit);
-            k_tea_force_partial<<<tg, kHiTile, 0, st>>>(Jp, a, j->jsplit);
-            k_tea_integrate<<<nb, kGridBlock, 0, st>>>(Jp, a, j->jsplit);
+            const int B = j->n <= kTeaOneBead ? 1 : 2;
+            cudaLaunchAttribute at;
+            const cudaLaunchConfig_t cfg = cluster_config(32 * kTeaWarps, kTeaCtas, (j->n + 32 * B - 1) / (32 * B), 0, st, &at);
+            CUDA_TRY(cudaLaunchKernelEx(&cfg, B == 1 ? k_tea_step<1> : k_tea_step<2>, Jp, a));
         } else {
             // the factor is refreshed every step (hi_refresh 1, the
             // reference) or at the updater boundaries due for it

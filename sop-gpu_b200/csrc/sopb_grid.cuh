@@ -23,7 +23,8 @@
 namespace sopb {
 
 constexpr int kGridBlock = 256;
-constexpr int kGridLpb = 4;
+constexpr int kGridLpb = 4;      // lanes per bead of the observables' sums
+constexpr int kForceLpb = 16;    // lanes per bead of k_g_forces
 constexpr int kCellMax = 1 << 22;
 constexpr int kSortCap = 2048;   // rows up to this length are sorted in registers
 
@@ -81,11 +82,12 @@ struct GridAux {
 __device__ __forceinline__ int64_t job_step(const JobDev* Jp) { return *(volatile const int64_t*)&Jp->step; }
 
 // ---- potentials ------------------------------------------------------------
-// Verlet-pair terms of bead i from its row (16-byte aligned), a 4-lane group:
-// lane l takes entries 4l..4l+3 of every 16 with one 16-byte load, and the
+// Verlet-pair terms of bead i from its row (16-byte aligned), a group of
+// kForceLpb lanes: lane l takes four entries with one 16-byte load, and the
 // next block's indices are fetched before this block's four gathers, so the
-// row load overlaps the coordinate gathers.
-static_assert(kGridLpb == 4, "one int4 of row entries per lane");
+// row load overlaps the coordinate gathers.  16 lanes, since only jobs with
+// hydrodynamics come here, which rarely fill the GPU: k_g_forces takes 9.0 us
+// at 517 beads and 9.5 at 4000 (14.4 and 16.1 with 4 lanes).
 __device__ __forceinline__ void pair_row_v4(const JobDev& J, const float4* __restrict__ xs,
                                             const int32_t* __restrict__ row, int cnt, float4 xi, int l, float3& f) {
     const float c8 = J.c8, cut2 = J.cut2;
@@ -93,9 +95,9 @@ __device__ __forceinline__ void pair_row_v4(const JobDev& J, const float4* __res
     int k = 4 * l;
     int4 nx = make_int4(0, 0, 0, 0);
     if (k < cnt) nx = __ldg(r4 + l);
-    for (; k < cnt; k += 16) {
+    for (; k < cnt; k += 4 * kForceLpb) {
         const int4 cur = nx;
-        if (k + 16 < cnt) nx = __ldg(r4 + (k >> 2) + 4);
+        if (k + 4 * kForceLpb < cnt) nx = __ldg(r4 + (k >> 2) + kForceLpb);
         if (k + 3 < cnt) {
             const float4 x0 = xs[cur.x], x1 = xs[cur.y], x2 = xs[cur.z], x3 = xs[cur.w];
             pair_term(xi, x0, c8, cut2, f);
@@ -163,7 +165,7 @@ k_g_forces(JobDev* __restrict__ Jp, GridAux aux) {
     __syncthreads();
     const JobDev& J = Js;
     if (J.status) return;
-    const int lpb = kGridLpb, l = threadIdx.x % lpb;
+    const int lpb = kForceLpb, l = threadIdx.x % lpb;
     const int groups = gridDim.x * (kGridBlock / lpb);
     const int g0 = blockIdx.x * (kGridBlock / lpb) + threadIdx.x / lpb;
     for (int base = 0; base < J.n; base += groups) {

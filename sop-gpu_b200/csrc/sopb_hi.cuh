@@ -1,12 +1,13 @@
 // sopb_hi.cuh — hydrodynamic interactions on the grid path.
 //
 // TEA (Geyer & Winter 2009, the reference's BDHI-TEA integrator,
-// src/Integrators/bdhitea_kernel.cu:192-515): the O(N^2) sums over all bead
-// pairs of a job run as tiles: a CTA takes 128 beads i and one slice of the
-// j range, stages the slice's coordinates and forces in shared memory
-// 128 at a time, and writes a partial sum per bead; a per-bead pass adds the
-// slices in slice order, so the result does not depend on scheduling.  The
-// per-job epsilon and beta' are reduced on the device in FP64, as the
+// src/Integrators/bdhitea_kernel.cu:192-515): a step's O(N^2) sums over all
+// bead pairs of a job and its move are one kernel (k_tea_step), a cluster of
+// CTAs per 32 or 64 beads.  The updater's sums run as tiles: a CTA takes 128
+// beads i and one slice of the j range, stages the slice's coordinates in
+// shared memory 128 at a time, and writes a partial sum per bead; a per-bead
+// pass adds the slices in slice order.  Either way the order of a sum does not
+// depend on scheduling.  The per-job epsilon and beta' are reduced on the device in FP64, as the
 // reference's host does (src/Integrators/bdhitea.cu:133-176).
 //
 // Exact HI for jobs up to 128 beads (3n <= 384, the reference's CHOLSIZE,
@@ -80,14 +81,27 @@ __device__ __forceinline__ void eps_stats(float4 xi, float4 xj, float a, float4&
     s.z += d.xz * d.xz + d.yz * d.yz + d.zz * d.zz;
 }
 
-// integrateTea_force (bdhitea_kernel.cu:252-301): D_ij (F_j + beta C_i o g_j).
-__device__ __forceinline__ void tea_pair(float4 xi, float4 xj, float4 mj, float4 rj, float3 bci, float a, float inv_a,
-                                         float3& f) {
-    const Blk6 d = rpy_fast(xi, xj, a, inv_a);
-    const float f0 = mj.x + rj.x * bci.x, f1 = mj.y + rj.y * bci.y, f2 = mj.z + rj.z * bci.z;
-    f.x += d.xx * f0 + d.xy * f1 + d.xz * f2;
-    f.y += d.xy * f0 + d.yy * f1 + d.yz * f2;
-    f.z += d.xz * f0 + d.yz * f1 + d.zz * f2;
+// integrateTea_force (bdhitea_kernel.cu:252-301): D_ij F with F = F_j + beta
+// C_i o g_j, as cii F + (crr / r^2) (d . F) d for the separation d: one
+// reciprocal square root, no unit vector and no block.
+struct TeaConst {
+    float far2, u1, c1, c2, n0, n1;
+    __device__ __forceinline__ explicit TeaConst(float a)
+        : far2(4.f * a * a), u1(0.75f * a), c1((2.f / 3.f) * a * a), c2(-2.f * a * a), n0((3.f / 32.f) / a), n1((-9.f / 32.f) / a) {}
+};
+__device__ __forceinline__ void tea_pair(float4 xi, float4 xj, float4 mj, float4 rj, float3 bci, const TeaConst& c, float3& f) {
+    const float dx = xj.x - xi.x, dy = xj.y - xi.y, dz = xj.z - xi.z;
+    const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+    const float ir = rsqrtf(r2), ir2 = ir * ir;
+    const bool far = r2 > c.far2;
+    const float u = c.u1 * ir;
+    const float cii = far ? u * fmaf(c.c1, ir2, 1.f) : fmaf(c.n1 * r2, ir, 1.f);
+    const float crr = far ? u * ir2 * fmaf(c.c2, ir2, 1.f) : c.n0 * ir;
+    const float f0 = fmaf(rj.x, bci.x, mj.x), f1 = fmaf(rj.y, bci.y, mj.y), f2 = fmaf(rj.z, bci.z, mj.z);
+    const float s = crr * fmaf(dx, f0, fmaf(dy, f1, dz * f2));
+    f.x = fmaf(cii, f0, fmaf(s, dx, f.x));
+    f.y = fmaf(cii, f1, fmaf(s, dy, f.y));
+    f.z = fmaf(cii, f2, fmaf(s, dz, f.z));
 }
 
 __device__ __forceinline__ bool tea_eps_due(const JobDev& J, int64_t step) {
@@ -193,81 +207,113 @@ __device__ __forceinline__ float3 tea_bci(const JobDev& J, const GridAux& aux, i
     return make_float3(ci.x * J.beta, ci.y * J.beta, ci.z * J.beta);
 }
 
-__global__ void __launch_bounds__(kHiTile)
-k_tea_force_partial(JobDev* __restrict__ Jp, GridAux aux, int jsplit) {
-    __shared__ float4 xs[kHiTile], ms[kHiTile], rs[kHiTile];
+// The sums and the move of a step.  A cluster of kTeaCtas CTAs takes 32 B
+// beads, each CTA a share of the partners (staged in shared memory kTeaChunk at
+// a time), each warp every eighth of those; a lane sums B beads, so the staged
+// operands are read once for B.  The partial sums go to the first CTA through
+// distributed shared memory and are added there in a fixed order (warps, then
+// CTAs), and that CTA moves the beads.
+// Bound by FP32 issue for large jobs: 31 us at 4000 beads (16 M pairs, 34
+// instructions each); 43 + 11 as tiles of 128 x 128 beads with the partial sums
+// in global memory and a second kernel that added them.  Below a thousand
+// beads one bead per lane gives every SM a CTA: 7.3 us at 517 beads, most of it
+// latency, where the tiles (25 CTAs) took 17 + 5.6.
+constexpr int kTeaCtas = 8, kTeaWarps = 8, kTeaChunk = 256;
+constexpr int kTeaOneBead = 1024;   // up to this size a lane sums one bead, above it two
+
+template <int B>
+__global__ void __launch_bounds__(32 * kTeaWarps)
+k_tea_step(JobDev* __restrict__ Jp, GridAux aux) {
+    __shared__ float4 stage[3][kTeaChunk > 32 * B * kTeaWarps / 3 ? kTeaChunk : 32 * B * kTeaWarps / 3 + 1];
+    __shared__ float4 sums[kTeaCtas][32 * B];
     const JobDev& J = *Jp;
     if (J.status) return;
-    const int n = J.n, i = blockIdx.x * kHiTile + threadIdx.x, s = blockIdx.y;
-    const float4 xi = aux.xc[i < n ? i : 0];
-    const float3 bci = tea_bci(J, aux, i < n ? i : 0, nullptr);
-    const float a = J.hi_a, inv_a = 1.f / J.hi_a;
-    float3 f = make_float3(0.f, 0.f, 0.f);
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");   // the other CTAs have begun
+    const int tid = threadIdx.x, l = tid & 31, w = tid >> 5, rank = blockIdx.x % kTeaCtas, i0 = blockIdx.x / kTeaCtas * (32 * B);
+    const int n = J.n;
+    float4 xi[B];
+    float3 bci[B], f[B];
+#pragma unroll
+    for (int b = 0; b < B; ++b) {
+        const int i = min(i0 + 32 * b + l, n - 1);
+        xi[b] = aux.xc[i];
+        bci[b] = tea_bci(J, aux, i, nullptr);
+        f[b] = make_float3(0.f, 0.f, 0.f);
+    }
+    const TeaConst c(J.hi_a);
     if (J.hi_unlisted) {
-        const int span = ((n + jsplit - 1) / jsplit + kHiTile - 1) / kHiTile * kHiTile;
-        const int j0 = s * span, j1 = min(n, j0 + span);
-        for (int t0 = j0; t0 < j1; t0 += kHiTile) {
+        const int span = (n + kTeaCtas - 1) / kTeaCtas, j0 = rank * span, j1 = min(n, j0 + span);
+        for (int t0 = j0; t0 < j1; t0 += kTeaChunk) {
+            const int cnt = min(kTeaChunk, j1 - t0);
             __syncthreads();
-            const int q = t0 + threadIdx.x;
-            if (q < j1) {
-                xs[threadIdx.x] = aux.xc[q];
-                ms[threadIdx.x] = aux.mf[q];
-                rs[threadIdx.x] = aux.rf[q];
+            for (int k = tid; k < cnt; k += 32 * kTeaWarps) {
+                stage[0][k] = aux.xc[t0 + k];
+                stage[1][k] = aux.mf[t0 + k];
+                stage[2][k] = aux.rf[t0 + k];
             }
             __syncthreads();
-            const int cnt = min(kHiTile, j1 - t0);
-            if (i < n) {
-                if (t0 == blockIdx.x * kHiTile) {   // the tile of this CTA's own beads
-                    for (int k = 0; k < cnt; ++k)
-                        if (t0 + k != i) tea_pair(xi, xs[k], ms[k], rs[k], bci, a, inv_a, f);
-                } else {
+            if (t0 < i0 + 32 * B && i0 < t0 + cnt) {   // some of the CTA's own beads
+                for (int k = w; k < cnt; k += kTeaWarps) {
+                    const float4 xj = stage[0][k], mj = stage[1][k], rj = stage[2][k];
+#pragma unroll
+                    for (int b = 0; b < B; ++b)
+                        if (t0 + k != i0 + 32 * b + l) tea_pair(xi[b], xj, mj, rj, bci[b], c, f[b]);
+                }
+            } else {
 #pragma unroll 4
-                    for (int k = 0; k < cnt; ++k) tea_pair(xi, xs[k], ms[k], rs[k], bci, a, inv_a, f);
+                for (int k = w; k < cnt; k += kTeaWarps) {
+                    const float4 xj = stage[0][k], mj = stage[1][k], rj = stage[2][k];
+#pragma unroll
+                    for (int b = 0; b < B; ++b) tea_pair(xi[b], xj, mj, rj, bci[b], c, f[b]);
                 }
             }
         }
-    } else if (s == 0 && i < n) {
-        // integrateTea_kernel: covalent, native and Verlet partners
-        for (int k = J.cov_off[i]; k < J.cov_off[i + 1]; ++k) {
-            const int q = J.cov_j[k];
-            tea_pair(xi, aux.xc[q], aux.mf[q], aux.rf[q], bci, a, inv_a, f);
-        }
-        for (int k = J.nat_off[i]; k < J.nat_off[i + 1]; ++k) {
-            const int q = J.nat_j[k];
-            tea_pair(xi, aux.xc[q], aux.mf[q], aux.rf[q], bci, a, inv_a, f);
-        }
-        const int32_t* row = J.pl_j + (size_t)i * J.cap_pl;
-        for (int k = 0; k < J.pl_cnt[i]; ++k) {
-            const int q = row[k];
-            tea_pair(xi, aux.xc[q], aux.mf[q], aux.rf[q], bci, a, inv_a, f);
+    } else {
+        // integrateTea_kernel: covalent, native and Verlet partners, every
+        // 64th of a list to a warp
+        const int first = rank * kTeaWarps + w, by = kTeaCtas * kTeaWarps;
+#pragma unroll
+        for (int b = 0; b < B; ++b) {
+            const int i = i0 + 32 * b + l;
+            if (i >= n) continue;
+            auto pair = [&](int q) { tea_pair(xi[b], aux.xc[q], aux.mf[q], aux.rf[q], bci[b], c, f[b]); };
+            for (int k = J.cov_off[i] + first; k < J.cov_off[i + 1]; k += by) pair(J.cov_j[k]);
+            for (int k = J.nat_off[i] + first; k < J.nat_off[i + 1]; k += by) pair(J.nat_j[k]);
+            const int32_t* row = J.pl_j + (size_t)i * J.cap_pl;
+            for (int k = first; k < J.pl_cnt[i]; k += by) pair(row[k]);
         }
     }
-    if (i < n) aux.part[(size_t)s * n + i] = make_float4(f.x, f.y, f.z, 0.f);
-}
-
-__global__ void __launch_bounds__(kGridBlock)
-k_tea_integrate(JobDev* __restrict__ Jp, GridAux aux, int jsplit) {
-    __shared__ JobDev Js;
-    load_job<kGridBlock>(Js, Jp);
+    // the warps' sums, then the CTAs'
     __syncthreads();
-    const JobDev& J = Js;
-    if (J.status) return;
-    const int n = J.n;
-    for (int i = blockIdx.x * kGridBlock + threadIdx.x; i < n; i += gridDim.x * kGridBlock) {
-        float3 ci;
-        tea_bci(J, aux, i, &ci);
-        const float4 m = aux.mf[i], r = aux.rf[i];
-        float3 f = make_float3(m.x + r.x * ci.x, m.y + r.y * ci.y, m.z + r.z * ci.z);
-        for (int s = 0; s < jsplit; ++s) {
-            const float4 p = aux.part[(size_t)s * n + i];
-            f.x += p.x; f.y += p.y; f.z += p.z;
+    float4* part = &stage[0][0];
+#pragma unroll
+    for (int b = 0; b < B; ++b) part[w * (32 * B) + 32 * b + l] = make_float4(f[b].x, f[b].y, f[b].z, 0.f);
+    __syncthreads();
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+    if (tid < 32 * B) {
+        float4 t = part[tid];
+        for (int q = 1; q < kTeaWarps; ++q) {
+            const float4 p = part[q * (32 * B) + tid];
+            t.x += p.x; t.y += p.y; t.z += p.z;
         }
-        if (J.pulling && J.flags[i] == FLAG_FIXED) f = make_float3(0.f, 0.f, 0.f);
-        const float4 xc = aux.xc[i];
-        const float dx = J.hOverZeta * f.x, dy = J.hOverZeta * f.y, dz = J.hOverZeta * f.z;
-        J.x[i] = make_float4(xc.x + dx, xc.y + dy, xc.z + dz, xc.w);
-        J.T[i] += J.tempNorm * (dx * dx + dy * dy + dz * dz);
+        const uint32_t to = map_rank((uint32_t)__cvta_generic_to_shared(&sums[rank][tid]), 0);
+        asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(to), "f"(t.x), "f"(t.y), "f"(t.z), "f"(t.w) : "memory");
     }
+    cluster_sync_all();
+    const int i = i0 + tid;
+    if (rank != 0 || tid >= 32 * B || i >= n) return;
+    float3 ci;
+    tea_bci(J, aux, i, &ci);
+    const float4 m = aux.mf[i], r = aux.rf[i], xc = aux.xc[i];
+    float3 F = make_float3(m.x + r.x * ci.x, m.y + r.y * ci.y, m.z + r.z * ci.z);
+    for (int q = 0; q < kTeaCtas; ++q) {
+        const float4 p = sums[q][tid];
+        F.x += p.x; F.y += p.y; F.z += p.z;
+    }
+    if (J.pulling && J.flags[i] == FLAG_FIXED) F = make_float3(0.f, 0.f, 0.f);
+    const float dx = J.hOverZeta * F.x, dy = J.hOverZeta * F.y, dz = J.hOverZeta * F.z;
+    J.x[i] = make_float4(xc.x + dx, xc.y + dy, xc.z + dz, xc.w);
+    J.T[i] += J.tempNorm * (dx * dx + dy * dy + dz * dz);
 }
 
 // ---- exact HI, n <= 128 ---------------------------------------------------------
