@@ -764,7 +764,7 @@ GridLayout grid_layout(const sopb_params& p, int64_t n, int sms, int64_t cap_pp,
     L.exact = L.hi && p.hi_exact;
     L.blocked = L.exact && n > 128;
     const int64_t itiles = (n + kHiTile - 1) / kHiTile;
-    if ((L.hi && !p.hi_exact && p.hi_unlisted) || L.blocked)
+    if (L.blocked)
         L.jsplit = (int)std::max<int64_t>(1, std::min<int64_t>((hi_cps * (int64_t)sms + itiles - 1) / itiles, itiles));
     size_t off = 0;
     auto take = [&](size_t bytes) { const size_t o = off; off += align256(bytes); return o; };
@@ -1102,9 +1102,9 @@ int grid_launch(sopb_job* j, cudaStream_t st, bool updaters, int steps, int due 
         if (a.cap_nr && (due & (kDuePossible | kDueVerlet))) k_g_near_commit<<<1, 32, 0, st>>>(Jp, a, -1, -1);
         if (j->h.hi && !j->h.hi_exact && (due & kDueTeaEps)) {
             // TeaUpdater (src/Integrators/bdhitea.cu:133-176), last updater
-            const dim3 tg((j->n + kHiTile - 1) / kHiTile, j->jsplit);
-            k_tea_eps_partial<<<tg, kHiTile, 0, st>>>(Jp, a, j->jsplit, 0);
-            k_tea_eps_reduce<<<nb, kGridBlock, 0, st>>>(Jp, a, j->jsplit, 0);
+            cudaLaunchAttribute at;
+            const cudaLaunchConfig_t cfg = cluster_config(32 * kTeaWarps, kTeaCtas, (j->n + 31) / 32, 0, st, &at);
+            CUDA_TRY(cudaLaunchKernelEx(&cfg, k_tea_eps, Jp, a, 0));
             k_tea_beta<<<1, 256, 0, st>>>(Jp, a, 0);
         }
     }
@@ -2327,7 +2327,8 @@ int current_context_id(unsigned long long* id) {
     return SOPB_ERR_CUDA;
 }
 
-// Unlisted branch of k_tea_eps_partial on plain pointers.
+// k_tea_eps's sums over all pairs on plain pointers, as tiles of 128 x 128
+// beads whose slices k_tea_eps_reduce_raw adds.
 __global__ void __launch_bounds__(kHiTile)
 k_tea_eps_partial_raw(const float4* __restrict__ x, int n, float a, int jsplit, float4* __restrict__ part) {
     __shared__ float4 xs[kHiTile];

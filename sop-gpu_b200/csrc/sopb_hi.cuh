@@ -1,14 +1,12 @@
 // sopb_hi.cuh — hydrodynamic interactions on the grid path.
 //
 // TEA (Geyer & Winter 2009, the reference's BDHI-TEA integrator,
-// src/Integrators/bdhitea_kernel.cu:192-515): a step's O(N^2) sums over all
-// bead pairs of a job and its move are one kernel (k_tea_step), a cluster of
-// CTAs per 32 or 64 beads.  The updater's sums run as tiles: a CTA takes 128
-// beads i and one slice of the j range, stages the slice's coordinates in
-// shared memory 128 at a time, and writes a partial sum per bead; a per-bead
-// pass adds the slices in slice order.  Either way the order of a sum does not
-// depend on scheduling.  The per-job epsilon and beta' are reduced on the device in FP64, as the
-// reference's host does (src/Integrators/bdhitea.cu:133-176).
+// src/Integrators/bdhitea_kernel.cu:192-515): the O(N^2) sums over all bead
+// pairs of a job, the step's (k_tea_step, which also moves the beads) and the
+// updater's (k_tea_eps), are taken by a cluster of CTAs per 32 or 64 beads, in
+// an order that does not depend on scheduling.  The per-job epsilon and beta'
+// are reduced on the device in FP64, as the reference's host does
+// (src/Integrators/bdhitea.cu:133-176).
 //
 // Exact HI for jobs up to 128 beads (3n <= 384, the reference's CHOLSIZE,
 // src/Integrators/bdhitea.h:24): the normalised RPY tensor D is assembled,
@@ -109,52 +107,64 @@ __device__ __forceinline__ bool tea_eps_due(const JobDev& J, int64_t step) {
 }
 
 // ---- TEA epsilon (updater) --------------------------------------------------
-__global__ void __launch_bounds__(kHiTile)
-k_tea_eps_partial(JobDev* __restrict__ Jp, GridAux aux, int jsplit, int force) {
-    __shared__ float4 xs[kHiTile];
+// The split of k_tea_step with a bead per lane.
+constexpr int kTeaCtas = 8, kTeaWarps = 8, kTeaChunk = 256;
+
+// The updater's sums.  Bound by FP32 issue for large jobs (a square root and
+// divisions per pair): 43 us at 4000 beads, 6.7 at 517 (latency); 47 + 10.5
+// and 20 + 5.2 as tiles of 128 x 128 beads and a second kernel that added the
+// slices.
+__global__ void __launch_bounds__(32 * kTeaWarps)
+k_tea_eps(JobDev* __restrict__ Jp, GridAux aux, int force) {
+    __shared__ float4 xs[kTeaChunk], part[kTeaWarps][32], sums[kTeaCtas][32];
     const JobDev& J = *Jp;
     const int64_t step = job_step(Jp);
     if (J.status || (!force && !tea_eps_due(J, step))) return;
-    const int n = J.n, i = blockIdx.x * kHiTile + threadIdx.x, s = blockIdx.y;
-    const float4 xi = J.x[i < n ? i : 0];
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");   // the other CTAs have begun
+    const int tid = threadIdx.x, l = tid & 31, w = tid >> 5, rank = blockIdx.x % kTeaCtas, i0 = blockIdx.x / kTeaCtas * 32;
+    const int n = J.n, i = i0 + l;
+    const float4 xi = J.x[min(i, n - 1)];
+    const float a = J.hi_a;
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
     if (J.hi_unlisted) {
-        const int span = ((n + jsplit - 1) / jsplit + kHiTile - 1) / kHiTile * kHiTile;
-        const int j0 = s * span, j1 = min(n, j0 + span);
-        for (int t0 = j0; t0 < j1; t0 += kHiTile) {
+        const int span = (n + kTeaCtas - 1) / kTeaCtas, j0 = rank * span, j1 = min(n, j0 + span);
+        for (int t0 = j0; t0 < j1; t0 += kTeaChunk) {
+            const int cnt = min(kTeaChunk, j1 - t0);
             __syncthreads();
-            if (t0 + threadIdx.x < j1) xs[threadIdx.x] = J.x[t0 + threadIdx.x];
+            if (tid < cnt) xs[tid] = J.x[t0 + tid];
             __syncthreads();
-            const int cnt = min(kHiTile, j1 - t0);
-            if (i < n)
-                for (int q = 0; q < cnt; ++q)
-                    if (t0 + q != i) eps_stats(xi, xs[q], J.hi_a, acc);
+            if (t0 < i0 + 32 && i0 < t0 + cnt) {       // some of the CTA's own beads
+                for (int k = w; k < cnt; k += kTeaWarps)
+                    if (t0 + k != i) eps_stats(xi, xs[k], a, acc);
+            } else {
+#pragma unroll 4
+                for (int k = w; k < cnt; k += kTeaWarps) eps_stats(xi, xs[k], a, acc);
+            }
         }
-    } else if (s == 0 && i < n) {
+    } else if (i < n) {
         // integrateTea_epsilon: covalent, native and Verlet partners
-        for (int k = J.cov_off[i]; k < J.cov_off[i + 1]; ++k) eps_stats(xi, J.x[J.cov_j[k]], J.hi_a, acc);
-        for (int k = J.nat_off[i]; k < J.nat_off[i + 1]; ++k) eps_stats(xi, J.x[J.nat_j[k]], J.hi_a, acc);
+        const int first = rank * kTeaWarps + w, by = kTeaCtas * kTeaWarps;
+        for (int k = J.cov_off[i] + first; k < J.cov_off[i + 1]; k += by) eps_stats(xi, J.x[J.cov_j[k]], a, acc);
+        for (int k = J.nat_off[i] + first; k < J.nat_off[i + 1]; k += by) eps_stats(xi, J.x[J.nat_j[k]], a, acc);
         const int32_t* row = J.pl_j + (size_t)i * J.cap_pl;
-        for (int k = 0; k < J.pl_cnt[i]; ++k) eps_stats(xi, J.x[row[k]], J.hi_a, acc);
+        for (int k = first; k < J.pl_cnt[i]; k += by) eps_stats(xi, J.x[row[k]], a, acc);
     }
-    if (i < n) aux.part[(size_t)s * n + i] = acc;
-}
-
-__global__ void __launch_bounds__(kGridBlock)
-k_tea_eps_reduce(JobDev* __restrict__ Jp, GridAux aux, int jsplit, int force) {
-    const JobDev& J = *Jp;
-    const int64_t step = job_step(Jp);
-    if (J.status || (!force && !tea_eps_due(J, step))) return;
-    const int n = J.n;
-    for (int i = blockIdx.x * kGridBlock + threadIdx.x; i < n; i += gridDim.x * kGridBlock) {
-        float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int s = 0; s < jsplit; ++s) {
-            const float4 p = aux.part[(size_t)s * n + i];
-            a.x += p.x; a.y += p.y; a.z += p.z; a.w += p.w;
-        }
-        aux.ci4[i] = a;
-        aux.eps[i] = a.w;
+    part[w][l] = acc;
+    __syncthreads();
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+    auto add4 = [](float4& t, float4 p) { t.x += p.x; t.y += p.y; t.z += p.z; t.w += p.w; };
+    if (tid < 32) {
+        float4 t = part[0][l];
+        for (int q = 1; q < kTeaWarps; ++q) add4(t, part[q][l]);
+        const uint32_t to = map_rank((uint32_t)__cvta_generic_to_shared(&sums[rank][l]), 0);
+        asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(to), "f"(t.x), "f"(t.y), "f"(t.z), "f"(t.w) : "memory");
     }
+    cluster_sync_all();
+    if (rank != 0 || tid >= 32 || i >= n) return;
+    float4 t = sums[0][l];
+    for (int q = 1; q < kTeaCtas; ++q) add4(t, sums[q][l]);
+    aux.ci4[i] = t;
+    aux.eps[i] = t.w;
 }
 
 // TeaUpdater::update's host arithmetic (bdhitea.cu:143-169) in FP64: the
@@ -218,7 +228,6 @@ __device__ __forceinline__ float3 tea_bci(const JobDev& J, const GridAux& aux, i
 // in global memory and a second kernel that added them.  Below a thousand
 // beads one bead per lane gives every SM a CTA: 7.3 us at 517 beads, most of it
 // latency, where the tiles (25 CTAs) took 17 + 5.6.
-constexpr int kTeaCtas = 8, kTeaWarps = 8, kTeaChunk = 256;
 constexpr int kTeaOneBead = 1024;   // up to this size a lane sums one bead, above it two
 
 template <int B>
