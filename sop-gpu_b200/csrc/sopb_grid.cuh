@@ -1018,7 +1018,7 @@ __device__ __forceinline__ bool in_sorted(const int32_t* row, int cnt, int v) {
 // Bound by latency: 206 us for the near rows of a 198000-bead shell (195
 // with a row per bead, which the step then gathers twice), 250 with one round's
 // gathers in flight.  A renewal of the near rows takes 1.6 ms
-// (0.56), mostly the searches; it is one of thousands of rebuilds.
+// (0.56), mostly the searches, and is rare next to the rebuilds from them.
 constexpr int kPairWarps = 4;      // warps per CTA
 constexpr int kPairBuf = 1024;     // entries of a possible row kept in shared memory for the searches
 constexpr int kPairTmp = 448;      // entries of a row that are near, before the searches

@@ -7,8 +7,8 @@ and retires finished ones (status, optional coordinates, asynchronous
 destroy), recording completion latency.
 
 Two kinds of job share the GPU:
-  - replica-resident jobs (no HI, up to 2048 beads): one CTA holds a whole
-    job, so they run best together, many jobs per launch;
+  - replica-resident jobs (no HI, up to 2048 beads): one CTA (a few
+    where SMs would idle) holds a whole job, so they run best together, many jobs per launch;
   - grid-path jobs (HI or above 2048 beads): chains of small launches.
 Resident jobs run in ragged launches of up to `batch_quantum` steps (each
 job's CTA stops at its own count) on a pool of highest-priority streams:
@@ -37,7 +37,7 @@ import numpy as np
 
 import sopb
 
-# jobs the library runs with the replica-resident kernel (one CTA per job)
+# jobs the library runs with the replica-resident kernel
 RESIDENT_MAX_BEADS = 2048
 
 
@@ -51,11 +51,12 @@ def step_cost(spec: "sopb.JobSpec") -> float:
     B200, which sizes a job's first quantum and orders jobs until its own
     quanta have been timed: a per-step launch chain, all-pairs O(n^2) sums
     for HI and, for exact HI, the factorisation amortised over its refresh
-    period -- up to 128 beads one CTA (about 0.023 n^2 us), above it the
+    period -- up to 128 beads one kernel (about 0.023 n^2 us), above it the
     chain of 3n/128 tile columns (about 3.8 n us) plus the O(n^2) apply --
     (fitted to 66 us per TEA step and 1.79 ms per exact step with refresh 10
     at 4000 beads, 71 and 224 us per exact step with refresh 1 at 40 and 90
-    beads), O(n) otherwise."""
+    beads, before the cluster kernels, which take 44 us per TEA step and 79 at
+    90 beads), O(n) otherwise."""
     p, n = spec.params, float(spec.n)
     if not p.hi_on:
         return 20.0 + 5e-4 * n
