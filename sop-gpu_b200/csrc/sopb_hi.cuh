@@ -120,7 +120,7 @@ k_tea_eps(JobDev* __restrict__ Jp, GridAux aux, int force) {
     const JobDev& J = *Jp;
     const int64_t step = job_step(Jp);
     if (J.status || (!force && !tea_eps_due(J, step))) return;
-    asm volatile("barrier.cluster.arrive.release;" ::: "memory");   // the other CTAs have begun
+    cluster_arrive();                                      // this CTA has begun: its shared memory may be written
     const int tid = threadIdx.x, l = tid & 31, w = tid >> 5, rank = blockIdx.x % kTeaCtas, i0 = blockIdx.x / kTeaCtas * 32;
     const int n = J.n, i = i0 + l;
     const float4 xi = J.x[min(i, n - 1)];
@@ -151,7 +151,7 @@ k_tea_eps(JobDev* __restrict__ Jp, GridAux aux, int force) {
     }
     part[w][l] = acc;
     __syncthreads();
-    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+    cluster_wait();
     auto add4 = [](float4& t, float4 p) { t.x += p.x; t.y += p.y; t.z += p.z; t.w += p.w; };
     if (tid < 32) {
         float4 t = part[0][l];
@@ -237,7 +237,7 @@ k_tea_step(JobDev* __restrict__ Jp, GridAux aux) {
     __shared__ float4 sums[kTeaCtas][32 * B];
     const JobDev& J = *Jp;
     if (J.status) return;
-    asm volatile("barrier.cluster.arrive.release;" ::: "memory");   // the other CTAs have begun
+    cluster_arrive();                                      // this CTA has begun: its shared memory may be written
     const int tid = threadIdx.x, l = tid & 31, w = tid >> 5, rank = blockIdx.x % kTeaCtas, i0 = blockIdx.x / kTeaCtas * (32 * B);
     const int n = J.n;
     float4 xi[B];
@@ -298,7 +298,7 @@ k_tea_step(JobDev* __restrict__ Jp, GridAux aux) {
 #pragma unroll
     for (int b = 0; b < B; ++b) part[w * (32 * B) + 32 * b + l] = make_float4(f[b].x, f[b].y, f[b].z, 0.f);
     __syncthreads();
-    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+    cluster_wait();
     if (tid < 32 * B) {
         float4 t = part[tid];
         for (int q = 1; q < kTeaWarps; ++q) {
@@ -644,6 +644,7 @@ k_hi_small(JobDev* __restrict__ Jp, GridAux aux, int refresh) {
     extern __shared__ __align__(16) float sm[];
     const JobDev& J = *Jp;
     if (J.status) return;                                   // the same for the whole cluster
+    cluster_arrive();                                       // this CTA has begun: its shared memory may be written
     const int C = (int)cluster_nctarank(), rank = (int)cluster_ctarank();
     const int n = J.n, m = 3 * n, T = small_blocks(n), ld = aux.ld;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -699,6 +700,10 @@ k_hi_small(JobDev* __restrict__ Jp, GridAux aux, int refresh) {
             }
         }
         __syncthreads();
+    }
+    // no CTA stores into another one that has not begun (the assembly hides the wait)
+    cluster_wait();
+    if (refresh) {
         if (rank == 0 && warp < kSmallDiagWarps) small_diag(rows, ldr, Dg, dinv, S, C, rank);
         for (int p = 0; p < T; ++p) {
             cluster_sync_all();                            // the factored tile is everywhere
