@@ -179,6 +179,7 @@ struct PartView {
     int cap;            // entries of nbr
     uint16_t* order;    // local pairs, longest row first (null in a cluster)
     float4* xref;       // coordinates the near list was built at, all beads
+    const int64_t* gave_up;   // step at which a chunk of steps that some CTA gave up ends
 };
 
 // A pair's row: `start` in the CTA's shared rows, or kRowGlobal for the
@@ -561,15 +562,39 @@ __device__ __forceinline__ bool peers_wait(uint32_t bar, uint32_t parity) {
     return false;
 }
 
+// A cluster gives up as a whole.  A CTA whose wait for its peers runs out
+// writes into every CTA's `gave_up` the step at which its chunk of steps ends,
+// arrives at its last cluster barrier and leaves.  The barrier that pairs with
+// it is the first one of an updater boundary at that step or later, or the last
+// one: a CTA there finds the step of its boundary reached and leaves as well,
+// without another barrier or a store into a peer, which may be gone.  A CTA
+// that gives up after the boundary writes a later step, so every thread that
+// looks sees the same, however late.  None writes its state back: the job keeps
+// the one it had at the launch (its lists may be newer), with the status
+// SOPB_ERR_TIMEOUT.
+constexpr int64_t kNeverStep = INT64_MAX;
+__device__ __forceinline__ int64_t gave_up_at(const int64_t* word) { return *(const volatile int64_t*)word; }
+__device__ __forceinline__ void give_up(int64_t* word, int C, int64_t step) {
+    if ((int)threadIdx.x < C) {
+        const uint32_t a = map_rank((uint32_t)__cvta_generic_to_shared(word), threadIdx.x);
+        asm volatile("st.relaxed.cluster.shared::cluster.b64 [%0], %1;" ::"r"(a), "l"(step) : "memory");
+    }
+}
+// A boundary's first cluster barrier; false when a peer gave up before it.
+__device__ __forceinline__ bool peers_meet(const PartView& V, int64_t step) {
+    cluster_sync_all();
+    return gave_up_at(V.gave_up) > step;
+}
+
 // Verlet rebuild of a resident job: from the near rows when they are valid
 // and no bead drifted more than half the skin from where they were built,
 // else a full scan that also renews the near rows at the current
 // coordinates.  The CTAs of a cluster decide alike: each looks at every bead
 // (its own copy of the coordinates and of x_ref), and after a full scan the
-// near rows count as valid when no CTA's overflowed.
+// near rows count as valid when no CTA's overflowed.  False when a peer gave up.
 template <bool CL>
-__device__ void rebuild_verlet(const JobDev& J, const PartView& V, const float4* __restrict__ xs, int& valid,
-                               bool possible_changed, int& err) {
+__device__ bool rebuild_verlet(const JobDev& J, const PartView& V, const float4* __restrict__ xs, int& valid,
+                               bool possible_changed, int64_t step, int& err) {
     __shared__ int drift_bits, near_over, alloc;
     const int tid = threadIdx.x, n = J.n;
     if (tid == 0) {
@@ -591,9 +616,9 @@ __device__ void rebuild_verlet(const JobDev& J, const PartView& V, const float4*
     __syncthreads();
     if (valid && !possible_changed && __int_as_float(drift_bits) < J.drift2) {
         build_verlet_near(J, V, &alloc, xs, err);
-        return;
+        return true;
     }
-    if (CL) cluster_sync_all();            // every CTA has cleared near_over
+    if (CL && !peers_meet(V, step)) return false;   // every CTA has cleared near_over
     build_verlet(J, V, &alloc, xs, err, &near_over);
     for (int i = tid; i < n; i += blockDim.x) V.xref[i] = xs[i];
     __syncthreads();
@@ -605,6 +630,7 @@ __device__ void rebuild_verlet(const JobDev& J, const PartView& V, const float4*
         cluster_sync_all();
     }
     valid = near_over || !(J.drift2 > 0.f) ? 0 : 1;   // drift2 0: the job keeps no near list
+    return true;
 }
 
 // Deterministic CTA sum of a float3 (fixed tree for a given BLOCK).
@@ -843,13 +869,13 @@ __device__ __noinline__ void store_rows(const JobDev& J, const PartView& V) {
 
 // The updaters of one `stride` boundary in the reference order
 // (creation order in src/gsop.cu:80-101; loop in src/gsop.cu:129-133).
-// Returns 1 when the Verlet list was rebuilt.
+// Returns 1 when the Verlet list was rebuilt, -1 when a peer gave up.
 template <bool CL>
 __device__ __noinline__ int run_updaters(const JobDev& J, const PartView& V, StepScalars& sc, const float4* __restrict__ xs,
                                          float* Ts, float (*red)[4], int64_t step, int& err) {
     const int tid = threadIdx.x, nb = V.b1 - V.b0;
     // the tip's and the plane's per-bead forces of the other CTAs' beads
-    if (CL && (J.indent || J.plane)) cluster_sync_all();
+    if (CL && (J.indent || J.plane) && !peers_meet(V, step)) return -1;
     if (J.indent) {
         if (tid == 0 && step == J.retraction_step) sc.V = -sc.V;
         if (step % J.nav == 0) {
@@ -886,7 +912,7 @@ __device__ __noinline__ int run_updaters(const JobDev& J, const PartView& V, Ste
     if (verlet) {
         if (pp) __syncthreads();
         int valid = sc.nr_valid;
-        rebuild_verlet<CL>(J, V, xs, valid, pp, err);
+        if (!rebuild_verlet<CL>(J, V, xs, valid, pp, step, err)) return -1;
         if (tid == 0) sc.nr_valid = valid;
         if (!CL) {
             __syncthreads();
@@ -926,12 +952,13 @@ k_resident_steps(JobDev* __restrict__ jobs, const int32_t* __restrict__ ids, con
     load_job(Js, Jp);
     __syncthreads();
     const JobDev& J = Js;
-    if (J.status != 0) return;             // the same for a job's CTAs: written after a cluster barrier
+    if (J.status != 0) return;             // the same for a job's CTAs: written after their last barrier
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ StepScalars sc;
     __shared__ PartView Vs;                // read as a broadcast, not held in registers
     __shared__ float red[32][4];
     __shared__ __align__(8) uint64_t bars[2];
+    __shared__ int64_t gave_up;
     __shared__ int next_task[2];           // per-step task counters, double buffered
     const int n = J.n, tid = threadIdx.x, lane = tid & 31, nt = blockDim.x;
     const int lc = 31 - __clz(C);          // C is a power of two
@@ -1005,7 +1032,8 @@ k_resident_steps(JobDev* __restrict__ jobs, const int32_t* __restrict__ ids, con
         sc.plane_displ = J.plane_displ;
         sc.plane_cant = J.plane_cant;
         Vs = PartView{p0, p1, b0, b1, rank, C, hdw, reinterpret_cast<uint16_t*>(smem + lay.nbr), J.lcache[lc], order,
-                      CL ? reinterpret_cast<float4*>(smem + lay.xref) : J.x_ref};
+                      CL ? reinterpret_cast<float4*>(smem + lay.xref) : J.x_ref, &gave_up};
+        gave_up = kNeverStep;
         if (CL) {
             for (int q = 0; q < 2; ++q)
                 asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"((uint32_t)__cvta_generic_to_shared(&bars[q])), "r"(1));
@@ -1033,11 +1061,19 @@ k_resident_steps(JobDev* __restrict__ jobs, const int32_t* __restrict__ ids, con
     const bool extra = J.indent || J.plane || J.discrete;
     int err = 0;
     bool built = false;
+    bool late = false, left = false;         // this CTA gave up; a peer did, and the last barrier is behind
     if (tid < 2) next_task[tid] = warps;
     __syncthreads();
     uint32_t s = 0;                          // steps of this launch, for the buffers' and mbarriers' parity
     while (step < last) {
-        if (phase == 0 && run_updaters<CL>(J, V, sc, xs, Ts, red, step, err)) built = true;
+        if (phase == 0) {
+            const int r = run_updaters<CL>(J, V, sc, xs, Ts, red, step, err);
+            if (CL && r < 0) {
+                left = true;
+                break;
+            }
+            if (r) built = true;
+        }
         int m = (int)min((int64_t)(J.stride - phase), last - step);   // steps to the next updater pass or the end
         step += m;
         phase = phase + m == J.stride ? 0 : phase + m;
@@ -1152,18 +1188,29 @@ k_resident_steps(JobDev* __restrict__ jobs, const int32_t* __restrict__ ids, con
             }
             if (CL) {
                 xs = xn;
-                const bool ok = peers_wait(bar, (s >> 1) & 1);
-                if (!__syncthreads_and(ok)) {
-                    err = SOPB_ERR_TIMEOUT;
+                if (!__syncthreads_and(peers_wait(bar, (s >> 1) & 1))) {
+                    late = true;
                     break;
                 }
             } else {
                 __syncthreads();
             }
         }
-        if (CL && err == SOPB_ERR_TIMEOUT) break;
+        if (CL && late) break;
     }
+    if (CL && late) give_up(&gave_up, C, step);
+    if (CL && !left) cluster_arrive();
     if (built) store_rows(J, V);
+    if (CL) {
+        if (!left) cluster_wait();           // none sends any more
+        if (gave_up_at(&gave_up) != kNeverStep) {
+            // the bytes of the step that was given up land before the shared memory is released
+            if (late) peers_wait((uint32_t)__cvta_generic_to_shared(&bars[s & 1]), (s >> 1) & 1);
+            if (tid == 0 && rank == 0) Jp->nr_valid = 0;   // near rows may have been renewed
+            if (tid == 0) atomicMax(&Jp->status, SOPB_ERR_TIMEOUT);
+            return;
+        }
+    }
     for (int b = tid; b < nb; b += nt) {
         const int i = b0 + b;
         const float4 v = xs[i];
@@ -1175,7 +1222,6 @@ k_resident_steps(JobDev* __restrict__ jobs, const int32_t* __restrict__ ids, con
     }
     if (err) atomicMax(&sc.err, err);
     __syncthreads();
-    if (CL) cluster_sync_all();               // every CTA has read the descriptor, none sends any more
     if (tid == 0) {
         if (rank == 0) {
             Jp->step = step;
@@ -1286,12 +1332,12 @@ k_rebuild_lists(JobDev* __restrict__ jobs, const int32_t* __restrict__ ids, int 
     if (threadIdx.x == 0) errs = 0;
     __syncthreads();
     int err = 0;
-    const PartView V{0, job_pairs(J.n), 0, J.n, 0, 1, nullptr, nullptr, 0, nullptr, J.x_ref};
+    const PartView V{0, job_pairs(J.n), 0, J.n, 0, 1, nullptr, nullptr, 0, nullptr, J.x_ref, nullptr};
     if (possible) build_possible(J, V, J.x, err);
     __syncthreads();
     if (verlet) {
         int valid = 0;                      // a full scan, which also renews the near list
-        rebuild_verlet<false>(J, V, J.x, valid, true, err);
+        rebuild_verlet<false>(J, V, J.x, valid, true, 0, err);
         if (threadIdx.x == 0) Jp->nr_valid = valid;
     } else if (possible && threadIdx.x == 0) {
         Jp->nr_valid = 0;                   // the near list no longer matches the possible pairs
