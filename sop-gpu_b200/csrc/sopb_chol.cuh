@@ -148,12 +148,15 @@ __device__ __forceinline__ void mma_f64(double2& c, double a, double b) {
 __global__ void __launch_bounds__(kPotrfThreads, 1)
 k_chol_potrf64(JobDev* __restrict__ Jp, GridAux aux, int J) {
     extern __shared__ __align__(16) double P64[];   // [kCT][kPotrfLd] the blocks
-    if (Jp->status) return;                         // read by every thread before any writes it (the barriers below)
+    __shared__ int stop;                            // read once: k_chol_tc on another stream may set the status
     double* Lp = P64 + kCT * kPotrfLd;              // [kCT][kPotrfLp] column k of L
     double* Xk = Lp + kCT * kPotrfLp;               // [kPotrfW][kPotrfLd] X's rows of step k
     constexpr int kWarps = kPotrfThreads / 32, kPer = kCT * kCT / 4 / kPotrfThreads;
     const int m = 3 * Jp->n, ld = aux.ld, base = J * kCT, nb = min(kCT, m - base);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, fr = lane >> 2, fc = lane & 3;
+    if (tid == 0) stop = Jp->status;
+    __syncthreads();
+    if (stop) return;
     float* M = aux.tensor + (size_t)base * ld + base;
     float* xout = aux.linv + (size_t)(J & 1) * kCT * kCT;   // two buffers: a solve may still read J - 1's
     {

@@ -331,12 +331,14 @@ k_g_step(JobDev* __restrict__ Jp, const GridAux aux, const float4* __restrict__ 
                 : "memory");
             there = ok;
         }
-        if (!__syncthreads_and(there)) {       // the copy did not arrive
-            if (tid == 0) atomicMax(&Jp->status, SOPB_ERR_TIMEOUT);
+        if (!__syncthreads_and(there && !status)) {
+            if (!there) atomicMax(&Jp->status, SOPB_ERR_TIMEOUT);   // the copy did not arrive
             return;
         }
     }
-    if (status) return;
+    // a narrow CTA voted, since another one may set the status meanwhile; no
+    // CTA of a wide step does, nor anything beside it on the job's stream
+    if (WIDE && status) return;
     const float cut2 = aux.cut2;
     const float3 zero = make_float3(0.f, 0.f, 0.f);
     float3 a0 = zero, a1 = zero, b0 = zero, b1 = zero, f = zero;
