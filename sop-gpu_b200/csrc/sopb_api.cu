@@ -1358,7 +1358,7 @@ extern "C" int sopb_job_create(sopb_context* c, const sopb_job_desc* d, sopb_job
     h.retraction_step = p.indentationRetractionStep;
     // force field constants as the reference hosts compute them
     h.ks = p.kspring_cov;
-    h.R2 = p.R_limit * p.R_limit;
+    h.R2 = std::min(p.R_limit * p.R_limit, kMaxR2);
     h.c8 = (float)(-6.0 * (double)p.el * std::pow((double)p.a, 6.0));
     h.cut2 = p.pairs_cutoff * p.pairs_cutoff;
     h.pl_cut = p.pairlist_cutoff;

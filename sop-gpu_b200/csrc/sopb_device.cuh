@@ -179,7 +179,8 @@ __device__ __forceinline__ float dist2_rn(float4 xi, float4 xj) {
 }
 __device__ __forceinline__ bool within_cutoff(float4 xi, float4 xj, float t) { return dist2_rn(xi, xj) < t; }
 
-// a / b for normal b and quotient: a reciprocal estimate refined by one
+// a / b for normal b and quotient (0 for |b| of 2^126 and more, whose reciprocal
+// is no normal number: a torn bond's denominator): a reciprocal estimate refined by one
 // Newton step, then the quotient corrected by its residual (P. Markstein,
 // "Computation of elementary functions on the IBM RISC System/6000
 // processor", 1990), within an ulp of the exact quotient.  It has no call and
@@ -191,11 +192,16 @@ __device__ __forceinline__ float div_newton(float a, float b) {
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b));
     r = fmaf(fmaf(-b, r, 1.0f), r, r);
     const float q = a * r;
-    return fmaf(fmaf(-b, q, a), r, q);
+    return fabsf(b) < 0x1p126f ? fmaf(fmaf(-b, q, a), r, q) : 0.0f;
 }
+// Largest R0^2 of the FENE term: its products with ks and the bond length stay
+// finite, and bonds shorter than 2^26 A do not tell it from a larger one (w^2 is
+// then below the last bit of R0^2).
+constexpr float kMaxR2 = 0x1p76f;
 
 // FENE term (covalent_kernel.cu:28-51): Ks*(r-r0)/(r*(1-(r-r0)^2/R0^2)),
-// numerator and denominator times R0^2 (one division).
+// numerator and denominator times R0^2 (one division); the host caps R0^2 at
+// kMaxR2.
 // r - r0 cancels for a near-relaxed bond, so r is formed with a correctly
 // rounded square root (the reference's fast-math build uses the approximate
 // one and loses ~1e-4 of the bond force there).
