@@ -444,7 +444,6 @@ k_chol_apply(JobDev* __restrict__ Jp, GridAux aux) {
 // L2 and took two barriers per column.
 constexpr int kSmallPanel = 32;
 constexpr int kSmallThreads = 512;
-constexpr int kSmallRows = 384;                            // 3n for n <= 128
 constexpr int kSmallMaxCtas = 8;
 constexpr int kSmallLdp = kSmallPanel + 4;                 // floats: rows of a panel, 16-byte aligned, no bank conflicts
 struct SmallLayout {                                       // in floats
@@ -475,7 +474,8 @@ __host__ __device__ inline SmallLayout small_layout(int n, int C) {
 }
 
 // 1 / sqrt(p): the hardware estimate and one Newton-Raphson step; d = sqrt(p)
-// by one residual correction.
+// by one residual correction (P. Markstein, "Computation of elementary functions
+// on the IBM RISC System/6000 processor", 1990); each within an ulp.
 __device__ __forceinline__ float rsqrt_newton(float p, float& d) {
     float y = rsqrtf(p);
     y = fmaf(0.5f * y, fmaf(-p * y, y, 1.0f), y);
@@ -483,7 +483,8 @@ __device__ __forceinline__ float rsqrt_newton(float p, float& d) {
     d = fmaf(fmaf(-d, d, p), 0.5f * y, d);
     return y;
 }
-// a / d from r ~ 1 / d, corrected by the quotient's residual
+// a / d from r ~ 1 / d, corrected by the quotient's residual (Markstein): within
+// an ulp
 __device__ __forceinline__ float quotient(float a, float d, float r) {
     const float q = a * r;
     return fmaf(fmaf(-q, d, a), r, q);
