@@ -10,6 +10,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <new>
 #include <vector>
@@ -2131,36 +2132,44 @@ extern "C" int sopb_job_pairlist(sopb_job* j, int32_t possible, int32_t* counts,
         // rows kept per pair of beads: both beads' partners, then each bead's
         // own, merged in increasing j
         const int32_t np = job_pairs(n), cap_u = j->h.cap_u, tile = j->h.mask ? 1 : j->h.tile;
-        const size_t slots = (size_t)(np + tile - 1) / tile * tile;
-        std::vector<int32_t> heads(4 * (size_t)np), rows_u(slots * cap_u);
-        if (j->h.mask) {
-            std::vector<uint2> vh(np);
-            std::vector<uint16_t> vr((size_t)np * cap_u);
-            CUDA_TRY(cudaMemcpyAsync(vh.data(), j->h.vh, vh.size() * sizeof(uint2), cudaMemcpyDeviceToHost, c->io));
-            CUDA_TRY(cudaMemcpyAsync(vr.data(), j->h.vr, vr.size() * 2, cudaMemcpyDeviceToHost, c->io));
-            SOPB_TRY(io_end(j, false));
-            for (int32_t p = 0; p < np; ++p) {
-                heads[4 * (size_t)p] = vh[p].y & 0xffff;
-                heads[4 * (size_t)p + 1] = vh[p].y >> 16;
-                heads[4 * (size_t)p + 2] = vh[p].x >> 20;
-                heads[4 * (size_t)p + 3] = 0;
+        std::vector<int32_t> row((size_t)cap_u);
+        auto merge = [&](const auto* vr, auto head) {
+            for (int32_t i = 0; i < n; ++i) {
+                const int4 hd = head(i >> 1);
+                const auto* r = vr + (size_t)((i >> 1) / tile) * tile * cap_u + hd.w;
+                const auto* own = r + hd.x + ((i & 1) ? hd.y : 0);
+                const auto *re = r + hd.x, *oe = own + ((i & 1) ? hd.z : hd.y);
+                int32_t* to = row.data();
+                for (; own != oe; ++own) {
+                    while (r != re && *r < *own) *to++ = *r++ >> 4;
+                    *to++ = *own >> 4;
+                }
+                while (r != re) *to++ = *r++ >> 4;
+                counts[i] = (int32_t)std::min<int64_t>(to - row.data(), j->h.cap_pl);
+                const int32_t len = std::max(std::min(counts[i], cap), 0);
+                std::copy_n(row.data(), len, rows + (size_t)i * cap);
+                std::fill(rows + (size_t)i * cap + len, rows + (size_t)i * cap + std::max(cap, 0), -1);
             }
-            std::copy(vr.begin(), vr.end(), rows_u.begin());
-        } else {
-            CUDA_TRY(cudaMemcpyAsync(heads.data(), j->h.gvh, heads.size() * 4, cudaMemcpyDeviceToHost, c->io));
-            CUDA_TRY(cudaMemcpyAsync(rows_u.data(), j->h.gvr, rows_u.size() * 4, cudaMemcpyDeviceToHost, c->io));
+        };
+        // (the copies' buffers are not filled first)
+        if (j->h.mask) {
+            const size_t nr = (size_t)np * cap_u;
+            std::unique_ptr<uint2[]> vh(new uint2[np]);
+            std::unique_ptr<uint16_t[]> vr(new uint16_t[nr]);
+            CUDA_TRY(cudaMemcpyAsync(vh.get(), j->h.vh, np * sizeof(uint2), cudaMemcpyDeviceToHost, c->io));
+            CUDA_TRY(cudaMemcpyAsync(vr.get(), j->h.vr, nr * 2, cudaMemcpyDeviceToHost, c->io));
             SOPB_TRY(io_end(j, false));
-        }
-        std::vector<int32_t> row;
-        for (int32_t i = 0; i < n; ++i) {
-            const int32_t* hd = heads.data() + 4 * (size_t)(i >> 1);
-            const int32_t* r = rows_u.data() + (size_t)((i >> 1) / tile) * tile * cap_u + hd[3];
-            const int32_t* own = r + hd[0] + ((i & 1) ? hd[1] : 0);
-            row.assign(r, r + hd[0]);
-            row.insert(row.end(), own, own + ((i & 1) ? hd[2] : hd[1]));
-            std::sort(row.begin(), row.end());
-            counts[i] = (int32_t)std::min<size_t>(row.size(), (size_t)j->h.cap_pl);
-            for (int32_t k = 0; k < cap; ++k) rows[(size_t)i * cap + k] = k < counts[i] ? row[k] >> 4 : -1;
+            merge(vr.get(), [&](int32_t p) {
+                return make_int4((int)(vh[p].y & 0xffff), (int)(vh[p].y >> 16), (int)(vh[p].x >> 20), 0);
+            });
+        } else {
+            const size_t nr = (size_t)(np + tile - 1) / tile * tile * cap_u;
+            std::unique_ptr<int4[]> vh(new int4[np]);
+            std::unique_ptr<int32_t[]> vr(new int32_t[nr]);
+            CUDA_TRY(cudaMemcpyAsync(vh.get(), j->h.gvh, np * sizeof(int4), cudaMemcpyDeviceToHost, c->io));
+            CUDA_TRY(cudaMemcpyAsync(vr.get(), j->h.gvr, nr * 4, cudaMemcpyDeviceToHost, c->io));
+            SOPB_TRY(io_end(j, false));
+            merge(vr.get(), [&](int32_t p) { return vh[p]; });
         }
         return SOPB_OK;
     }

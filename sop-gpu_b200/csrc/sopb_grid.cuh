@@ -61,7 +61,7 @@ struct GridAux {
     int32_t* nr_j;       // [n * cap_nr] possible pairs within pairlist_cutoff + skin
     int32_t* nr_cnt;     // [n]
     float4* x_ref;       // coordinates it was built at
-    int32_t* near;       // [3] drift bits, overflow, usable
+    int32_t* near;       // [4] drift bits, overflow, usable, not tried again
     int32_t cap_nr;
     // Verlet rows per pair of beads of a job without hydrodynamics (whose near
     // rows are per pair as well: nr_j and nr_cnt by pair)
@@ -877,10 +877,17 @@ static_assert(kSortCap == 2048, "k_cl_sort_rows handles rows up to 32 x 64 keys 
 // was closer than pairlist_cutoff + skin then, so filtering the near rows with
 // the same exact test gives the rows a filter of the possible rows gives.
 // aux.near: [0] largest squared drift (float bits), [1] a near row overflowed
-// its capacity, [2] the near list is usable.  [0] and [1] are cleared by
-// k_g_near_commit, the last kernel of every rebuild.
+// its capacity, [2] the near list is usable, [3] it overflowed since the
+// possible pairs are what they are: it would again, and rebuilds filter the
+// possible rows without trying (jobs without hydrodynamics).  [0] and [1] are
+// cleared by k_g_near_commit, the last kernel of every rebuild.
 __device__ __forceinline__ bool verlet_from_near(const JobDev& J, const GridAux& a, int64_t step, int force) {
     return !force && a.nr_j && a.near[2] && step % J.pp_freq != 0 && __int_as_float(a.near[0]) < J.drift2;
+}
+
+// Whether a rebuild that is not from the near rows renews them.
+__device__ __forceinline__ bool near_renewed(const JobDev& J, const GridAux& a, int64_t step, int force) {
+    return a.nr_j && (force || !a.vh || !a.near[3] || step % J.pp_freq == 0);
 }
 
 // Largest squared displacement since the near list was built, at a Verlet
@@ -991,60 +998,151 @@ k_g_verlet(JobDev* __restrict__ Jp, GridAux a, int force) {
     if (over) atomicOr(&a.near[1], 1);
 }
 
-// Whether a sorted row of cnt entries holds v.
-__device__ __forceinline__ bool in_sorted(const int32_t* row, int cnt, int v) {
-    int lo = 0, hi = cnt;
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (row[mid] < v) lo = mid + 1;
-        else hi = mid;
-    }
-    return lo < cnt && row[lo] == v;
-}
-
 // Verlet rows (pairlist_kernel.cu:33-76) of a job without hydrodynamics, per
 // pair of beads (2p, 2p + 1): the partners of both, of the first alone, of the
-// second alone.  A warp per pair.
-// Candidates are 8 q with bit 0 when the first bead may pair with q and bit 1
-// when the second may, in this order: the first bead's possible partners
-// (increasing j; a search in the second bead's row gives bit 1), then those of
-// the second bead that are not the first one's.  The near rows hold the
-// candidates within pairlist_cutoff + skin of a bead they may pair with, in
-// the same order, so a rebuild from them places the same hits in the same
-// order as one from all candidates.
-// As in the resident kernel, ballots give each hit its place in its section
-// (kept in a register for the first eight rounds of 32), then the hits are
-// stored.  More than max_pairs partners of a bead sets err.
+// second alone, each in increasing j.  A warp per pair.
+// A bead's partners are its possible partners (increasing j) within the cutoff.
+// The warp filters both beads' possible rows into shared memory, a part at a
+// time, and merges the two: what both lists hold is a partner of both.  The near
+// rows are merged in the same way from what is within pairlist_cutoff + skin,
+// as 8 q with bit 0 when q is near the first bead and bit 1 when it is near the
+// second; a rebuild from them tests their entries alone.  Either way a row's
+// sections come out in increasing j.
+// As in the resident kernel, ballots give each hit its place in its section,
+// then the hits are stored.  More than max_pairs partners of a bead sets err.
 // A CTA takes a tile of pairs at a time and gives their rows consecutive places
 // (any order: a header holds its row's start), four rounds' gathers in flight.
-// Bound by latency: 206 us for the near rows of a 198000-bead shell (195
-// with a row per bead, which the step then gathers twice), 250 with one round's
-// gathers in flight.  A renewal of the near rows takes 1.6 ms
-// (0.56), mostly the searches, and is rare next to the rebuilds from them.
-constexpr int kPairWarps = 4;      // warps per CTA
-constexpr int kPairBuf = 1024;     // entries of a possible row kept in shared memory for the searches
-constexpr int kPairTmp = 448;      // entries of a row that are near, before the searches
-__device__ __forceinline__ int pair_hit(const float4* __restrict__ x, float4 x0, float4 x1, float t, int e) {
-    const float4 q = x[e >> 3];
-    return ((dist2_rn(x0, q) < t ? 1 : 0) | (dist2_rn(x1, q) < t ? 2 : 0)) & e;
+// Bound by latency: 169 us from the near rows of a 198000-bead shell, 566 when
+// they are renewed (192 and 552 with a row per bead, which the step then gathers
+// twice; 1600 when a near entry was searched for in the other bead's row).  200
+// steps of 6000 beads without near rows 2.0 ms, 2.6 with a row per bead (3.3 with
+// searches; 32 when the possible rows hold all beads).  Eight warps: a tile's 32
+// pairs four deep (18000 beads without near rows 3.1 ms, 3.8 with four warps);
+// three CTAs per SM: 80 registers without a spill (64 slow the near rebuilds).
+constexpr int kPairWarps = 8;      // warps per CTA
+constexpr int kPairBuf = 512;      // entries of a filtered possible row kept in shared memory
+
+// The possible partners of a bead within the root of t, increasing, from
+// `o` to `n` of a warp's buffer; the row's entries from k on are still to come.
+struct Filtered {
+    const int32_t* row;
+    int cnt, k, o, n;
+    int32_t* buf;
+    float4 x;
+};
+// At least 32 entries or all there are.
+__device__ __forceinline__ void refill(Filtered& f, const float4* __restrict__ x, float t) {
+    if (f.k >= f.cnt || f.n - f.o >= 32) return;
+    const int l = threadIdx.x & 31, left = f.n - f.o;
+    const unsigned below = (1u << l) - 1u;
+    const int keep = l < left ? f.buf[f.o + l] : 0;
+    __syncwarp();
+    if (l < left) f.buf[l] = keep;
+    int n = left, k = f.k, nq[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) nq[u] = f.row[min(k + 32 * u + l, f.cnt - 1)];
+    for (; k < f.cnt && n + 128 <= kPairBuf; k += 128) {
+        int q[4];
+        float4 xq[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            q[u] = nq[u];
+            xq[u] = x[q[u]];
+        }
+        // the next entries while these ones' coordinates are on the way
+#pragma unroll
+        for (int u = 0; u < 4; ++u) nq[u] = f.row[min(k + 128 + 32 * u + l, f.cnt - 1)];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const bool in = k + 32 * u + l < f.cnt && dist2_rn(f.x, xq[u]) < t;
+            const unsigned m = __ballot_sync(0xffffffffu, in);
+            if (in) f.buf[n + __popc(m & below)] = q[u];
+            n += __popc(m);
+        }
+    }
+    f.o = 0;
+    f.n = n;
+    f.k = k;
+    __syncwarp();
 }
-template <typename Cand>
-__device__ __forceinline__ void build_pair_row(const JobDev& J, const GridAux& a, int p, float4 x0, float4 x1, int rounds,
-                                               Cand cand, int* alloc, int& err) {
+// Entries of the warp's sorted window (a lane each) below v.
+__device__ __forceinline__ int window_rank(int w, int v) {
+    int r = 0;
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1)
+        if (__shfl_sync(0xffffffffu, w, r + s - 1) < v) r += s;
+    return r + (__shfl_sync(0xffffffffu, w, r) < v ? 1 : 0);
+}
+// Merges two filtered rows, up to 32 entries of each at a time: visit(a, bits
+// of a, b, bits of b, a's rank in the second window, the second window's
+// entries that are in the first).  Bits 3 for an entry of both (once, as a), 1
+// and 2 for one of the first or second alone, 0 for none.
+template <typename Visit>
+__device__ __forceinline__ void merge_rows(Filtered& A, Filtered& B, const float4* __restrict__ x, float t, Visit visit) {
+    const int l = threadIdx.x & 31;
+    const unsigned all = 0xffffffffu;
+    constexpr int kEnd = 0x7fffffff;
+    for (;;) {
+        refill(A, x, t);
+        refill(B, x, t);
+        const int na = A.n - A.o, nb = B.n - B.o;
+        if (na + nb == 0) break;
+        const int a = l < na ? A.buf[A.o + l] : kEnd, b = l < nb ? B.buf[B.o + l] : kEnd;
+        // as far as both windows are complete
+        const int enda = na > 32 || A.k < A.cnt ? __shfl_sync(all, a, 31) : kEnd;
+        const int endb = nb > 32 || B.k < B.cnt ? __shfl_sync(all, b, 31) : kEnd;
+        const int end = min(enda, endb);
+        const bool ta = l < na && a <= end, tb = l < nb && b <= end;
+        const int r = window_rank(b, a);
+        const bool both = __shfl_sync(all, b, r & 31) == a && ta && r < 32;
+        const unsigned dup = __reduce_or_sync(all, both ? 1u << r : 0u);
+        visit(a, ta ? (both ? 3 : 1) : 0, b, tb && !((dup >> l) & 1u) ? 2 : 0, r, dup);
+        A.o += __popc(__ballot_sync(all, ta));
+        B.o += __popc(__ballot_sync(all, tb));
+    }
+}
+
+// Room for pair p's row and its header: sections of nf, n0 and n1 entries, cut
+// off where a bead has more than max_pairs partners.
+struct PairRow {
+    int32_t* dst;
+    int nf, n0, n1;
+    __device__ __forceinline__ void store(int hit, int pos, int entry) const {
+        pos += hit == 3 ? 0 : (hit == 1 ? nf : nf + n0);
+        if (hit && pos < nf + n0 + n1) dst[pos] = entry;
+    }
+};
+__device__ __forceinline__ PairRow place_row(const JobDev& J, const GridAux& a, int p, int nf, int n0, int n1, int* alloc, int& err) {
     const int l = threadIdx.x & 31, cap = a.cap_u & ~3;
+    if (max(n0, n1) + nf > J.cap_pl) {
+        err = SOPB_STATUS_CAPACITY;
+        nf = min(nf, cap);
+        n0 = min(n0, cap - nf);
+        n1 = min(n1, cap - nf - n0);
+    }
+    int start = 0;
+    if (a.tile > 1) {
+        if (l == 0) start = atomicAdd(alloc, (nf + n0 + n1 + 3) & ~3);
+        start = __shfl_sync(0xffffffffu, start, 0);
+    }
+    if (l == 0) a.vh[p] = make_int4(nf, n0, n1, start);
+    return {a.vr + (size_t)(p / a.tile) * a.tile * a.cap_u + start, nf, n0, n1};
+}
+
+// Pair p's row from its near row.
+__device__ __forceinline__ void row_from_near(const JobDev& J, const GridAux& a, int p, float4 x0, float4 x1, const int32_t* nrow,
+                                              int count, int* alloc, int& err) {
+    const int l = threadIdx.x & 31, rounds = (count + 31) >> 5;
     const unsigned below = (1u << l) - 1u, all = 0xffffffffu;
     int cf = 0, c0 = 0, c1 = 0;
-    auto take = [&](int hit) {
+    auto cand = [&](int u) { return 32 * u + l < count ? nrow[32 * u + l] : 0; };
+    auto take = [&](float4 q, int e, int& at) {
+        const int hit = ((dist2_rn(x0, q) < J.pl_t ? 1 : 0) | (dist2_rn(x1, q) < J.pl_t ? 2 : 0)) & e;
         const unsigned mf = __ballot_sync(all, hit == 3), m0 = __ballot_sync(all, hit == 1), m1 = __ballot_sync(all, hit == 2);
-        const int at = (hit == 3 ? cf : (hit == 1 ? c0 : c1)) + __popc((hit == 3 ? mf : (hit == 1 ? m0 : m1)) & below);
+        at = (hit == 3 ? cf : (hit == 1 ? c0 : c1)) + __popc((hit == 3 ? mf : (hit == 1 ? m0 : m1)) & below);
         cf += __popc(mf);
         c0 += __popc(m0);
         c1 += __popc(m1);
-        return at;
-    };
-    auto round = [&](int e, int& at) {
-        const int hit = pair_hit(J.x, x0, x1, J.pl_t, e);
-        at = take(hit);
         return (e & ~7) | hit;
     };
     int w[kKeptRounds], place[kKeptRounds];
@@ -1058,108 +1156,81 @@ __device__ __forceinline__ void build_pair_row(const JobDev& J, const GridAux& a
 #pragma unroll
             for (int v = 0; v < 4; ++v) q[v] = J.x[w[u + v] >> 3];
 #pragma unroll
-            for (int v = 0; v < 4; ++v) {
-                const int hit = ((dist2_rn(x0, q[v]) < J.pl_t ? 1 : 0) | (dist2_rn(x1, q[v]) < J.pl_t ? 2 : 0)) & w[u + v];
-                w[u + v] = (w[u + v] & ~7) | hit;
-                place[u + v] = take(hit);
-            }
+            for (int v = 0; v < 4; ++v) w[u + v] = take(q[v], w[u + v], place[u + v]);
         }
     const int kf = cf, k0 = c0, k1 = c1;
     int at;
-    for (int u = kKeptRounds; u < rounds; ++u) round(cand(u), at);
-    int nf = cf, n0 = c0, n1 = c1;
-    if (max(n0, n1) + nf > J.cap_pl) {
-        err = SOPB_STATUS_CAPACITY;
-        nf = min(nf, cap);
-        n0 = min(n0, cap - nf);
-        n1 = min(n1, cap - nf - n0);
+    for (int u = kKeptRounds; u < rounds; ++u) {
+        const int e = cand(u);
+        take(J.x[e >> 3], e, at);
     }
-    const int len = nf + n0 + n1;
-    int start = 0;
-    if (a.tile > 1) {
-        if (l == 0) start = atomicAdd(alloc, (len + 3) & ~3);
-        start = __shfl_sync(all, start, 0);
-    }
-    int32_t* dst = a.vr + (size_t)(p / a.tile) * a.tile * a.cap_u + start;
-    auto store = [&](int v, int pos) {
-        const int hit = v & 3;
-        pos += hit == 3 ? 0 : (hit == 1 ? nf : nf + n0);
-        if (hit && pos < len) dst[pos] = 2 * (v & ~7);       // 16 j
-    };
+    const PairRow row = place_row(J, a, p, cf, c0, c1, alloc, err);
 #pragma unroll
     for (int u = 0; u < kKeptRounds; ++u)
-        if (u < rounds) store(w[u], place[u]);
+        if (u < rounds) row.store(w[u] & 3, place[u], 2 * (w[u] & ~7));       // 16 j
     cf = kf;
     c0 = k0;
     c1 = k1;
     for (int u = kKeptRounds; u < rounds; ++u) {
-        const int v = round(cand(u), at);
-        store(v, at);
+        const int e = cand(u), v = take(J.x[e >> 3], e, at);
+        row.store(v & 3, at, 2 * (v & ~7));
     }
-    if (l == 0) a.vh[p] = make_int4(nf, n0, n1, start);
 }
 
-// The near row of pair p: its candidates within nr_t of a bead they may pair
-// with.  First the entries of a possible row that are near at all, then the
-// searches in the other row for those.
-__device__ __forceinline__ int build_near_row(const JobDev& J, int32_t* nrow, int cap, const int32_t* s0, int c0, const int32_t* s1,
-                                              int c1, float4 x0, float4 x1, int32_t* tmp) {
+// Pair p's row from the possible rows of its beads.
+__device__ __forceinline__ void row_from_possible(const JobDev& J, const GridAux& a, int p, const Filtered& A0, const Filtered& B0,
+                                                  int* alloc, int& err) {
+    const unsigned below = (1u << (threadIdx.x & 31)) - 1u, all = 0xffffffffu;
+    int cf = 0, c0 = 0, c1 = 0;
+    auto pass = [&](Filtered A, Filtered B, auto store) {
+        cf = c0 = c1 = 0;
+        merge_rows(A, B, J.x, J.pl_t, [&](int qa, int ba, int qb, int bb, int, unsigned) {
+            const unsigned mf = __ballot_sync(all, ba == 3), m0 = __ballot_sync(all, ba == 1), m1 = __ballot_sync(all, bb);
+            store(ba, (ba == 3 ? cf + __popc(mf & below) : c0 + __popc(m0 & below)), 16 * qa);
+            store(bb, c1 + __popc(m1 & below), 16 * qb);
+            cf += __popc(mf);
+            c0 += __popc(m0);
+            c1 += __popc(m1);
+        });
+    };
+    Filtered A = A0, B = B0;
+    refill(A, J.x, J.pl_t);
+    refill(B, J.x, J.pl_t);
+    const bool whole = A.k >= A.cnt && B.k >= B.cnt;    // both stay as they are for the second pass
+    pass(A, B, [](int, int, int) {});
+    const PairRow row = place_row(J, a, p, cf, c0, c1, alloc, err);
+    pass(whole ? A : A0, whole ? B : B0, [&](int hit, int pos, int entry) { row.store(hit, pos, entry); });
+}
+
+// The near row of pair p; its length, also beyond its capacity.
+__device__ __forceinline__ int build_near_row(const JobDev& J, int32_t* nrow, int cap, Filtered A, Filtered B) {
     const int l = threadIdx.x & 31;
     const unsigned below = (1u << l) - 1u, all = 0xffffffffu;
     int count = 0;
-    for (int h = 0; h < 2; ++h) {
-        const int32_t* own = h ? s1 : s0;
-        const int32_t* other = h ? s0 : s1;
-        const int cown = h ? c1 : c0, cother = h ? c0 : c1;
-        for (int kb = 0; kb < cown;) {
-            // up to kPairTmp near entries of the row
-            int m = 0;
-            for (; kb < cown && m + 128 <= kPairTmp; kb += 128) {
-                int q[4];
-                float4 xq[4];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) q[u] = own[min(kb + 32 * u + l, cown - 1)];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) xq[u] = J.x[q[u]];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    unsigned bits = (dist2_rn(x0, xq[u]) < J.nr_t ? 1u : 0u) | (dist2_rn(x1, xq[u]) < J.nr_t ? 2u : 0u);
-                    if (h) bits &= 2u;
-                    if (kb + 32 * u + l >= cown) bits = 0;
-                    const unsigned v = __ballot_sync(all, bits != 0);
-                    if (bits) tmp[m + __popc(v & below)] = 8 * q[u] + (int)bits;
-                    m += __popc(v);
-                }
-            }
-            __syncwarp();
-            for (int k = 0; k < m; k += 32) {
-                int e = k + l < m ? tmp[k + l] : 0;
-                // of the first row: bit 1 stands if the second one holds it
-                // too; of the second row: only what the first one does not hold
-                if (!h && (e & 2) && !in_sorted(other, cother, e >> 3)) e &= ~2;
-                if (h && e && in_sorted(other, cother, e >> 3)) e = 0;
-                const unsigned v = __ballot_sync(all, e & 3);
-                const int pos = count + __popc(v & below);
-                if ((e & 3) && pos < cap) nrow[pos] = e;
-                count += __popc(v);
-            }
-            __syncwarp();
-        }
-    }
+    merge_rows(A, B, J.x, J.nr_t, [&](int qa, int ba, int qb, int bb, int r, unsigned dup) {
+        const unsigned ma = __ballot_sync(all, ba), mb = __ballot_sync(all, bb);
+        // before a: the lanes below and the second row's own entries below its rank
+        const unsigned lower = r < 32 ? (1u << r) - 1u : all;
+        const int pa = count + l + __popc(mb & lower);
+        if (ba && pa < cap) nrow[pa] = 8 * qa + ba;
+        const int pb = count + __popc(mb & below) + window_rank(qa, qb);
+        if (bb && pb < cap) nrow[pb] = 8 * qb + 2;
+        count += __popc(ma) + __popc(mb);
+    });
     return count;
 }
 
-__global__ void __launch_bounds__(32 * kPairWarps)
+__global__ void __launch_bounds__(32 * kPairWarps, 3)
 k_g_pair_rows(JobDev* __restrict__ Jp, GridAux a, int force) {
     __shared__ JobDev Js;
-    __shared__ int32_t buf[kPairWarps][2][kPairBuf], tmp[kPairWarps][kPairTmp];
+    __shared__ int32_t buf[kPairWarps][2][kPairBuf];
     __shared__ int alloc;
     load_job<32 * kPairWarps>(Js, Jp);
     __syncthreads();
     const JobDev& J = Js;
     const int64_t step = J.step;
     if (J.status || (!force && (step % J.stride != 0 || step % J.pairs_freq != 0))) return;
-    const bool near = verlet_from_near(J, a, step, force);
+    const bool near = verlet_from_near(J, a, step, force), renew = !near && near_renewed(J, a, step, force);
     const int l = threadIdx.x & 31, wp = threadIdx.x >> 5, np = (J.n + 1) >> 1;
     const int group = max(a.tile, kPairWarps), groups = (np + group - 1) / group;
     int err = 0, over = 0;
@@ -1172,48 +1243,25 @@ k_g_pair_rows(JobDev* __restrict__ Jp, GridAux a, int force) {
             int32_t* nrow = a.nr_j ? a.nr_j + (size_t)p * a.cap_nr : nullptr;
             int count = near ? a.nr_cnt[p] : 0;
             bool from_near = near;
-            int c0 = 0, c1 = 0;
-            const int32_t *s0 = nullptr, *s1 = nullptr;
+            Filtered A, B;
             if (!near) {
-                c0 = J.pp_cnt[2 * p];
-                c1 = two ? J.pp_cnt[2 * p + 1] : 0;
-                const int32_t *r0 = J.pp_j + (size_t)(2 * p) * J.cap_pp, *r1 = r0 + J.cap_pp;
-                s0 = r0;
-                s1 = r1;
-                if (c0 <= kPairBuf) {
-                    for (int k = l; k < c0; k += 32) buf[wp][0][k] = r0[k];
-                    s0 = buf[wp][0];
+                const int32_t* r0 = J.pp_j + (size_t)(2 * p) * J.cap_pp;
+                A = {r0, J.pp_cnt[2 * p], 0, 0, 0, buf[wp][0], x0};
+                B = {r0 + J.cap_pp, two ? J.pp_cnt[2 * p + 1] : 0, 0, 0, 0, buf[wp][1], x1};
+            }
+            if (renew) {
+                count = build_near_row(J, nrow, a.cap_nr, A, B);
+                if (l == 0) {
+                    a.nr_cnt[p] = min(count, a.cap_nr);
+                    a.x_ref[2 * p] = x0;
+                    if (two) a.x_ref[2 * p + 1] = x1;
                 }
-                if (c1 <= kPairBuf) {
-                    for (int k = l; k < c1; k += 32) buf[wp][1][k] = r1[k];
-                    s1 = buf[wp][1];
-                }
+                if (count > a.cap_nr) over = 1;
+                else from_near = true;
                 __syncwarp();
-                if (nrow) {
-                    count = build_near_row(J, nrow, a.cap_nr, s0, c0, s1, c1, x0, x1, tmp[wp]);
-                    if (l == 0) {
-                        a.nr_cnt[p] = min(count, a.cap_nr);
-                        a.x_ref[2 * p] = x0;
-                        if (two) a.x_ref[2 * p + 1] = x1;
-                    }
-                    if (count > a.cap_nr) over = 1;
-                    else from_near = true;
-                    __syncwarp();
-                }
             }
-            if (from_near) {
-                build_pair_row(J, a, p, x0, x1, (count + 31) >> 5,
-                               [&](int u) { return 32 * u + l < count ? nrow[32 * u + l] : 0; }, &alloc, err);
-            } else {
-                // no near row: straight from the candidates
-                const int rounds0 = (c0 + 31) >> 5;
-                auto cand = [&](int u) {
-                    const int k = 32 * (u < rounds0 ? u : u - rounds0) + l;
-                    if (u < rounds0) return k < c0 ? 8 * s0[k] + 1 + (in_sorted(s1, c1, s0[k]) ? 2 : 0) : 0;
-                    return k < c1 && !in_sorted(s0, c0, s1[k]) ? 8 * s1[k] + 2 : 0;
-                };
-                build_pair_row(J, a, p, x0, x1, rounds0 + ((c1 + 31) >> 5), cand, &alloc, err);
-            }
+            if (from_near) row_from_near(J, a, p, x0, x1, nrow, count, &alloc, err);
+            else row_from_possible(J, a, p, A, B, &alloc, err);
             __syncwarp();
         }
         __syncthreads();
@@ -1238,9 +1286,16 @@ __global__ void k_g_near_commit(JobDev* __restrict__ Jp, GridAux a, int possible
         possible = at && step % J.pp_freq == 0;
         verlet = at && step % J.pairs_freq == 0;
     }
-    if (J.status) a.near[2] = 0;
-    else if (verlet && !verlet_from_near(J, a, step, force ? 1 : 0)) a.near[2] = a.near[1] ? 0 : 1;
-    else if (possible && !verlet) a.near[2] = 0;
+    if (J.status) {
+        a.near[2] = 0;
+    } else if (verlet && !verlet_from_near(J, a, step, force ? 1 : 0)) {
+        const bool renewed = near_renewed(J, a, step, force ? 1 : 0);
+        a.near[2] = renewed && !a.near[1] ? 1 : 0;
+        if (renewed) a.near[3] = a.near[1] ? 1 : 0;
+    } else if (possible && !verlet) {
+        a.near[2] = 0;
+        a.near[3] = 0;
+    }
     a.near[0] = 0;
     a.near[1] = 0;
 }
