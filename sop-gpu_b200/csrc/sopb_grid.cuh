@@ -202,15 +202,21 @@ k_g_forces(JobDev* __restrict__ Jp, GridAux aux) {
 // after another, arrive in shared memory by one bulk copy while the bonded
 // terms are computed.
 //
-// Measured per step (free globules, 20 A lists, rebuilds included): 5011 beads
-// 9.5 us wide, 15.3 narrow; 20000 beads 16.6 and 18.8; 30000 beads 20.8 and
-// 19.0 -- the line lies between.  A clamped chain of 5011 beads takes 10.7 us
-// per step, 14.0 with a lane group per bead and the integrator as a kernel of
-// its own (whose forces and moves took 16.0 + 5.1 us under the profiler, this
-// kernel 12.0); a 198000-bead shell 106 us, 126 before (88 + 6 us, now 70).
-constexpr int kWideStepBeads = 24576;   // up to this size the step takes wide groups
+// Wide CTAs take 32 beads, and three of them fit an SM (80 registers): up to
+// 148 x 3 x 32 = 14208 beads they run in one wave.  Above, narrow steps are
+// faster (per step of 200, rebuilds included; clamped globules, 20 A lists):
+// 12000 beads 10.7 us wide, 14.3 narrow; 18000 beads 15.6 and 13.4, a shell of
+// 18000 beads 15.8 and 10.9; 24000 beads 17.2 and 15.1.  With a lane group per
+// bead and the integrator as a kernel of its own: 14.4, 15.8, 14.8 and 18.5.
+// A clamped chain of 5011 beads takes 10.5 us per step, 14.0 before; a
+// 198000-bead shell 102 us, 126 before (88 + 6 us under the profiler, now 70).
+constexpr int kWideStepBeads = 14208;
 __host__ __device__ constexpr int step_pairs(bool wide) { return kGridBlock / (wide ? 16 : 8); }   // pairs per CTA
-constexpr int kStepRow = 192;           // row entries per pair that a CTA has shared memory for
+// Row entries per pair that a CTA has shared memory for: four CTAs' share of an
+// SM.  A tile whose rows are longer reads them from global memory (40000 beads
+// with 26 and 32 A lists: 15.1 and 21.9 us per step, 20.0 and 32.5 with a lane
+// group per bead).
+constexpr int kStepRow = 192;
 constexpr uint32_t kStepWaitLimit = 1u << 20;
 
 // Entries [k0 + l, k1) of a row in steps of G, four gathers in flight:
