@@ -11,6 +11,7 @@
 #include <cstring>
 #include <map>
 #include <memory>
+#include <queue>
 #include <mutex>
 #include <new>
 #include <vector>
@@ -116,6 +117,9 @@ struct LaunchClass {
 // uploading again.
 struct RunPlan {
     uint64_t generation = 0;
+    int share = 1;                // streams that shared the GPU when it was made
+    cudaEvent_t done = nullptr;   // the stream's last run ended (a context with runs on several streams)
+    uint64_t overlap = 0;         // the context's run count when a run was last seen beside one on this stream
     std::vector<sopb_job*> jobs;
     std::vector<int64_t> steps;
     std::vector<LaunchClass> cls;
@@ -131,6 +135,7 @@ struct sopb_context {
     int sm_count = 0;
     uint64_t generation = 0;      // bumped by every job creation and destruction
     std::map<cudaStream_t, RunPlan> plans;   // the last resident launch plan per stream
+    uint64_t runs = 0;            // runs with resident jobs
     int64_t bead_cap = 0;
     float4* x = nullptr;
     float4* xalt = nullptr;
@@ -570,6 +575,8 @@ extern "C" int sopb_context_destroy(sopb_context* c) {
         }
         cudaEventDestroy(f.fork);
     }
+    for (auto& kv : c->plans)
+        if (kv.second.done) cudaEventDestroy(kv.second.done);
     cudaStreamDestroy(c->capture);
     cudaStreamDestroy(c->upload);
     cudaStreamDestroy(c->io);
@@ -1733,44 +1740,120 @@ int ctas_per_sm(const sopb_context* c, int block, size_t smem) {
 // CTAs per job of a run of resident jobs (log2, per job).  With one CTA per
 // job a run ends with its largest job, and one of fewer jobs than SMs leaves
 // SMs idle.  So the job that would take longest doubles its CTAs as long as
-// the run's CTAs have an SM each, within what clusters of that size reach,
-// or -- with enough jobs to fill the SMs anyway -- the job takes longer than
-// the run's work spread over all SMs (200 replicas of 60 to 600 beads: 3.0 ms
-// per 200 steps, 4.7 without); a CTA keeps at least kClusterMinBeads beads.  A step of n beads on C CTAs takes about
-// n / C bead times, plus the cluster's exchange, worth kClusterBeads beads
-// (200 steps of 600 beads: 3.5 ms on one CTA, 0.9 ms on sixteen).  A job's
-// arithmetic does not depend on its cluster.
+// the run's CTAs have an SM each, within what clusters of that size reach; a
+// CTA keeps at least kClusterMinBeads beads.  A step of n beads on C CTAs takes
+// about n / C bead times, plus the cluster's exchange, worth kClusterBeads beads
+// (200 steps of 600 beads: 3.5 ms on one CTA, 0.9 ms on sixteen).  With enough
+// jobs to fill the SMs anyway a job still doubles while it takes longer than the
+// run's work spread over all SMs, where run_span says that the run ends earlier:
+// 100 steps of 200 replicas of 60 to 600 beads 1.8 ms, 2.1 without; but 119
+// equal jobs of 200 beads 1.18 and 0.99.  Last, no job keeps more CTAs than a
+// larger one has with which the run ends.  A run beside runs on other streams
+// (`share` of them in all) plans with its share of the SMs: 100 steps of four
+// streams of 10 jobs of 200 beads each take 0.84 ms, 1.35 when each run plans for
+// the whole GPU; eight streams of 20 jobs 1.39 and 2.99.
+// A job's arithmetic does not depend on its cluster.
 constexpr int kClusterMinBeads = 12;
 constexpr double kClusterBeads = 12.0;
-std::vector<int> cluster_sizes(const sopb_context* c, sopb_job* const* jobs, int32_t njobs) {
-    std::vector<int> lc((size_t)njobs, 0);
+constexpr double kBesideCost = 0.725;   // of a single CTA's time on an SM that another one shares (148 jobs of
+                                        // 200 beads 1.79 ms per 200 steps, 296 of them 2.6)
+double cluster_cost(const sopb_job* j, int lc) { return (double)j->n / (1 << lc) + (lc ? kClusterBeads : 0.0); }
+
+// The time a run takes by these costs when its CTAs go longest first to the SM
+// that is free first.
+double run_span(sopb_job* const* jobs, int32_t njobs, const std::vector<int>& lc, int sms) {
+    std::vector<std::pair<double, int>> ctas;   // cost, CTAs per job
+    for (int32_t j = 0; j < njobs; ++j) ctas.insert(ctas.end(), (size_t)1 << lc[j], {cluster_cost(jobs[j], lc[j]), lc[j]});
+    std::sort(ctas.begin(), ctas.end(), [](auto& a, auto& b) { return a.first > b.first; });
+    std::priority_queue<double, std::vector<double>, std::greater<double>> sm;
+    for (int k = 0; k < sms; ++k) sm.push(0.0);
+    double end = 0.0;
+    for (auto& t : ctas) {
+        const double at = sm.top();
+        sm.pop();
+        sm.push(at + (t.second || at == 0.0 ? t.first : kBesideCost * t.first));
+        end = std::max(end, at + t.first * (t.second || at == 0.0 ? 1.0 : kBesideCost));
+    }
+    return end;
+}
+
+std::vector<int> cluster_sizes(const sopb_context* c, sopb_job* const* jobs, int32_t njobs, int share) {
+    std::vector<int> lc((size_t)njobs, 0), filled;
+    const int sms = std::max(1, c->sm_count / share);
     int64_t used = njobs;
     double work = 0.0;
     for (int32_t j = 0; j < njobs; ++j) work += jobs[j]->n;
-    auto cost = [&](int32_t j) { return (double)jobs[j]->n / (1 << lc[j]) + (lc[j] ? kClusterBeads : 0.0); };
+    int32_t worst;
     for (;;) {
-        int32_t worst = 0;
+        worst = 0;
         for (int32_t j = 1; j < njobs; ++j)
-            if (cost(j) > cost(worst)) worst = j;
+            if (cluster_cost(jobs[j], lc[j]) > cluster_cost(jobs[worst], lc[worst])) worst = j;
         const int k = lc[worst];
-        if (k + 1 >= kClusterSizes || !c->cluster_ctas[k + 1] || (jobs[worst]->n >> (k + 1)) < kClusterMinBeads) return lc;
-        const bool one_wave = used + (1 << k) <= c->cluster_ctas[k + 1];
-        if (!one_wave && (k >= 2 || 5 * njobs < 4 * c->sm_count || cost(worst) < 1.15 * work / c->sm_count)) return lc;
+        if (k + 1 >= kClusterSizes || !c->cluster_ctas[k + 1] || (jobs[worst]->n >> (k + 1)) < kClusterMinBeads) break;
+        const bool one_wave = used + (1 << k) <= std::min(sms, c->cluster_ctas[k + 1]);
+        if (!one_wave) {
+            if (k >= 2 || 5 * njobs < 4 * sms || cluster_cost(jobs[worst], k) < 1.15 * work / sms) break;
+            if (filled.empty()) filled = lc;
+        }
         lc[worst] = k + 1;
         used += 1 << k;
         work += kClusterBeads * (k ? 1 << k : 2);
     }
+    if (!filled.empty() && run_span(jobs, njobs, filled, sms) <= run_span(jobs, njobs, lc, sms)) {
+        lc = filled;
+        for (int32_t j = 0; j < njobs; ++j)
+            if (cluster_cost(jobs[j], lc[j]) > cluster_cost(jobs[worst], lc[worst])) worst = j;
+    }
+    for (int32_t j = 0; j < njobs; ++j)
+        if (jobs[j]->n <= jobs[worst]->n) lc[j] = std::min(lc[j], lc[worst]);
+    return lc;
+}
+
+bool capturing(cudaStream_t st) {
+    cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &s) != cudaSuccess) cudaGetLastError();
+    return s != cudaStreamCaptureStatusNone;
+}
+
+// How many streams share the GPU with a run on `st`: those whose runs were seen
+// beside another one's within the last 64 runs, if this stream's were too.
+// (Queries are allowed beside a stream capture only in the relaxed mode.)
+int streams_sharing(sopb_context* c, cudaStream_t st, RunPlan& plan) {
+    ++c->runs;
+    if (c->plans.size() < 2) return 1;
+    if (capturing(st)) return plan.share;   // the plan at hand needs no upload
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    for (auto& kv : c->plans) {
+        if (kv.first == st || !kv.second.done || kv.second.jobs.empty()) continue;
+        const cudaError_t e = cudaEventQuery(kv.second.done);
+        if (e != cudaSuccess) cudaGetLastError();   // not an error of this call
+        if (e == cudaErrorNotReady) kv.second.overlap = plan.overlap = c->runs;
+    }
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    int share = 1;
+    if (plan.overlap && c->runs - plan.overlap <= 64)
+        for (auto& kv : c->plans)
+            if (kv.first != st && kv.second.overlap && c->runs - kv.second.overlap <= 64 && !kv.second.jobs.empty()) ++share;
+    return share;
+}
+// Marks the end of a run on `st` for streams_sharing.
+int run_ended(sopb_context* c, cudaStream_t st, RunPlan& plan) {
+    if (c->plans.size() < 2 || capturing(st)) return SOPB_OK;
+    if (!plan.done) CUDA_TRY(cudaEventCreateWithFlags(&plan.done, cudaEventDisableTiming));
+    CUDA_TRY(cudaEventRecord(plan.done, st));
+    return SOPB_OK;
 }
 
 // Jobs of one class share the lanes per bead, a cluster size, a CTA size and the number of CTAs
 // an SM holds, so the class's largest shared-memory request never lowers the
 // residency of its smaller jobs.
-void group_jobs(const sopb_context* c, sopb_job* const* jobs, int32_t njobs, std::vector<LaunchClass>& out) {
+void group_jobs(const sopb_context* c, sopb_job* const* jobs, int32_t njobs, int share, std::vector<LaunchClass>& out) {
     std::map<int, LaunchClass> cls;   // key: (lanes per bead, wide, cluster; CTA size, CTAs per SM)
     std::vector<int32_t> order(njobs);
     for (int32_t k = 0; k < njobs; ++k) order[k] = k;
     std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) { return jobs[a]->n > jobs[b]->n; });
-    const std::vector<int> lc = cluster_sizes(c, jobs, njobs);
+    const std::vector<int> lc = cluster_sizes(c, jobs, njobs, share);
     for (int32_t k : order) {
         const JobDev& h = jobs[k]->h;
         const int lg = lc[k], C = 1 << lg;
@@ -1867,14 +1950,23 @@ int run_ordered(sopb_context* c, sopb_job* const* jobs, int32_t njobs, const int
     const std::vector<LaunchClass>& cls = plan.cls;
     const std::vector<size_t>& off = plan.off;
     if (!resident.empty()) {
-        const bool same = plan.generation == c->generation && plan.jobs == resident && plan.steps == rsteps;
+        const int share = streams_sharing(c, st, plan);
+        const bool same = plan.generation == c->generation && plan.jobs == resident && plan.steps == rsteps && plan.share == share;
         if (!same) {
+            plan.share = share;
             plan.generation = c->generation;
             plan.jobs = resident;
             plan.steps = rsteps;
             plan.cls.clear();
             plan.off.clear();
-            group_jobs(c, resident.data(), (int32_t)resident.size(), plan.cls);
+            group_jobs(c, resident.data(), (int32_t)resident.size(), 1, plan.cls);
+            // runs of several classes queue on the side streams: each has the
+            // GPU to itself in turn (four streams of 40 jobs of 60 to 600 beads
+            // 4.1 ms per 100 steps, 7.8 with shares); one class is beside the others
+            if (share > 1 && plan.cls.size() == 1) {
+                plan.cls.clear();
+                group_jobs(c, resident.data(), (int32_t)resident.size(), share, plan.cls);
+            }
         }
         std::vector<int64_t> slot_steps(c->slots.size(), 0);
         for (size_t k = 0; k < resident.size(); ++k) slot_steps[resident[k]->slot] = rsteps[k];
@@ -1893,8 +1985,10 @@ int run_ordered(sopb_context* c, sopb_job* const* jobs, int32_t njobs, const int
             CUDA_TRY(cudaMemcpyAsync(d_ids, ids.data(), ids.size() * 4, cudaMemcpyHostToDevice, st));
             CUDA_TRY(cudaMemcpyAsync(d_steps, steps.data(), steps.size() * 8, cudaMemcpyHostToDevice, st));
         }
-        if (grid.empty() && cls.size() == 1)
-            return launch_resident(cls[0], st, c->d_jobs, d_ids, d_steps);
+        if (grid.empty() && cls.size() == 1) {
+            SOPB_TRY(launch_resident(cls[0], st, c->d_jobs, d_ids, d_steps));
+            return run_ended(c, st, plan);
+        }
     } else {
         // no resident jobs in this run: no classes to launch, and the table
         // on this stream is no longer the plan's
@@ -1930,7 +2024,7 @@ int run_ordered(sopb_context* c, sopb_job* const* jobs, int32_t njobs, const int
         CUDA_TRY(cudaEventRecord(f->gjoin[k], f->gside[k]));
         CUDA_TRY(cudaStreamWaitEvent(st, f->gjoin[k], 0));
     }
-    return SOPB_OK;
+    return resident.empty() ? SOPB_OK : run_ended(c, st, plan);
 }
 }  // namespace
 
