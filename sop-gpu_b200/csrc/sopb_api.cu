@@ -344,14 +344,19 @@ int launch_resident(const LaunchClass& L, cudaStream_t st, JobDev* jobs, const i
     return SOPB_OK;
 }
 
-int launch_forces(int block, int grid, cudaStream_t st, const JobDev* jobs, const int32_t* ids, float4* out) {
-    k_forces_only<<<grid, block, 0, st>>>(jobs, ids, out);
+// One job's forces, its lane groups over as many CTAs as they fill.
+int launch_forces(const sopb_context* c, const JobDev& h, cudaStream_t st, const int32_t* ids, float4* out) {
+    const int ctas = (int)std::min<int64_t>(((int64_t)h.n * h.lpb + h.block - 1) / h.block, c->sm_count);
+    k_forces_only<<<dim3(1, ctas), h.block, 0, st>>>(c->d_jobs, ids, out);
     CUDA_TRY(cudaGetLastError());
     return SOPB_OK;
 }
 
-int launch_rebuild(int block, int grid, cudaStream_t st, JobDev* jobs, const int32_t* ids, int possible, int verlet) {
-    k_rebuild_lists<<<grid, block, 0, st>>>(jobs, ids, possible, verlet);
+// One resident job's lists, by a cluster of CTAs.
+int launch_rebuild(const sopb_context* c, const JobDev& h, cudaStream_t st, const int32_t* ids, int possible, int verlet) {
+    cudaLaunchAttribute at;
+    const cudaLaunchConfig_t cfg = cluster_config(h.block, rebuild_ctas(h.n), 1, 0, st, &at);
+    CUDA_TRY(cudaLaunchKernelEx(&cfg, k_rebuild_lists, c->d_jobs, ids, possible, verlet));
     CUDA_TRY(cudaGetLastError());
     return SOPB_OK;
 }
@@ -2091,7 +2096,7 @@ extern "C" int sopb_job_read(sopb_job* j, int32_t what, void* out) {
         if (rc) return rc;
         const int32_t id = j->slot;
         CUDA_TRY(cudaMemcpyAsync(d_ids, &id, 4, cudaMemcpyHostToDevice, c->io));
-        rc = launch_forces(j->h.block, 1, c->io, c->d_jobs, d_ids, c->d_scratch4);
+        rc = launch_forces(c, j->h, c->io, d_ids, c->d_scratch4);
         if (rc) return rc;
         CUDA_TRY(cudaMemcpyAsync(out, c->d_scratch4, n * 16, cudaMemcpyDeviceToHost, c->io));
         break;
@@ -2306,7 +2311,7 @@ extern "C" int sopb_job_rebuild_lists(sopb_job* j, int32_t possible, int32_t ver
     if (rc) return rc;
     const int32_t id = j->slot;
     CUDA_TRY(cudaMemcpyAsync(d_ids, &id, 4, cudaMemcpyHostToDevice, c->io));
-    rc = launch_rebuild(j->h.block, 1, c->io, c->d_jobs, d_ids, possible, verlet);
+    rc = launch_rebuild(c, j->h, c->io, d_ids, possible, verlet);
     if (rc) return rc;
     SOPB_TRY(io_end(j, true));
     return SOPB_OK;

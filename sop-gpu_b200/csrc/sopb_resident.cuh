@@ -1247,7 +1247,8 @@ k_resident_steps(JobDev* __restrict__ jobs, const int32_t* __restrict__ ids, con
 
 // Potential forces only (SOPPotential::compute of every potential, no
 // integrator) at the job's current coordinates and Verlet rows, with the
-// step kernel's lane split; does not touch the tip accumulator.
+// step kernel's lane split; does not touch the tip accumulator.  blockIdx.y
+// shares a job's beads.
 __global__ void __launch_bounds__(1024, 1)
 k_forces_only(const JobDev* __restrict__ jobs, const int32_t* __restrict__ ids, float4* __restrict__ out) {
     __shared__ JobDev Js;
@@ -1263,7 +1264,7 @@ k_forces_only(const JobDev* __restrict__ jobs, const int32_t* __restrict__ ids, 
     IndentGeom ig;
     for (int c = 0; c < 3; ++c) { ig.tip[c] = J.tip[c]; ig.micaR[c] = J.micaR[c]; ig.micaN[c] = J.micaN[c]; }
     ig.tipR = J.tipR; ig.tipAp = J.tipAp; ig.tipBp = J.tipBp; ig.surfAp = J.surfAp; ig.surfBp = J.surfBp;
-    for (int base = 0; base < tasks; base += ng) {
+    for (int base = blockIdx.y * ng; base < tasks; base += gridDim.y * ng) {
         const int t = base + tid / G, i = pairs ? 2 * t + h : t;
         const bool act = i < n;
         const float4 xi = J.x[act ? i : 0];
@@ -1321,27 +1322,36 @@ k_forces_only(const JobDev* __restrict__ jobs, const int32_t* __restrict__ ids, 
     }
 }
 
-// Rebuilds the possible-pairs and/or Verlet lists now, without the step gate.
+// Rebuilds the possible-pairs and/or Verlet lists of a job now, without the step
+// gate: a cluster of CTAs with a share of its pairs each.  Bound by latency: a
+// call that renews the Verlet rows of 600 beads takes 59 us, of 2000 beads 285
+// (130 and 945 with one CTA and a row per bead; 200 and 2010 with one CTA).
+__host__ __device__ inline int rebuild_ctas(int n) { return n >= 256 ? 8 : (n >= 64 ? 4 : 1); }
 __global__ void __launch_bounds__(1024, 1)
 k_rebuild_lists(JobDev* __restrict__ jobs, const int32_t* __restrict__ ids, int possible, int verlet) {
-    JobDev* Jp = &jobs[ids[blockIdx.x]];
+    const int C = (int)cluster_nctarank(), rank = (int)cluster_ctarank();
+    JobDev* Jp = &jobs[ids[blockIdx.x / C]];
     __shared__ JobDev Js;
     load_job(Js, Jp);
     const JobDev& J = Js;
     __shared__ int errs;
-    if (threadIdx.x == 0) errs = 0;
+    __shared__ int64_t gave_up;
+    cluster_arrive();                        // this CTA has begun: its shared memory may be written
+    if (threadIdx.x == 0) {
+        errs = 0;
+        gave_up = kNeverStep;
+    }
     __syncthreads();
     int err = 0;
-    const PartView V{0, job_pairs(J.n), 0, J.n, 0, 1, nullptr, nullptr, 0, nullptr, J.x_ref, nullptr};
+    const int p0 = pair_begin(J.n, rank, C), p1 = pair_begin(J.n, rank + 1, C);
+    const PartView V{p0, p1, 2 * p0, min(J.n, 2 * p1), rank, C, nullptr, nullptr, 0, nullptr, J.x_ref, &gave_up};
     if (possible) build_possible(J, V, J.x, err);
     __syncthreads();
-    if (verlet) {
-        int valid = 0;                      // a full scan, which also renews the near list
-        rebuild_verlet<false>(J, V, J.x, valid, true, 0, err);
-        if (threadIdx.x == 0) Jp->nr_valid = valid;
-    } else if (possible && threadIdx.x == 0) {
-        Jp->nr_valid = 0;                   // the near list no longer matches the possible pairs
-    }
+    cluster_wait();
+    int valid = 0;
+    if (verlet) rebuild_verlet<true>(J, V, J.x, valid, true, 0, err);   // a full scan, which also renews the near list
+    // (without it the near list no longer matches the possible pairs)
+    if ((verlet || possible) && rank == 0 && threadIdx.x == 0) Jp->nr_valid = valid;
     if (err) atomicMax(&errs, err);
     __syncthreads();
     if (threadIdx.x == 0 && errs) Jp->status = errs;

@@ -70,7 +70,7 @@ def late_waits(fns):
 
 def test_cluster_kernels_wait_for_their_peers_first():
     found, bad = late_waits(functions())
-    assert found == ["k_hi_small", "k_resident_steps", "k_tea_eps", "k_tea_step"]
+    assert found == ["k_hi_small", "k_rebuild_lists", "k_resident_steps", "k_tea_eps", "k_tea_step"]
     assert bad == []
 
 
