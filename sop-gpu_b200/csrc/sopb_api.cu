@@ -1859,6 +1859,8 @@ void group_jobs(const sopb_context* c, sopb_job* const* jobs, int32_t njobs, int
     for (int32_t k = 0; k < njobs; ++k) order[k] = k;
     std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) { return jobs[a]->n > jobs[b]->n; });
     const std::vector<int> lc = cluster_sizes(c, jobs, njobs, share);
+    // a run without clusters of no more jobs than SMs
+    const bool roomy = (int64_t)njobs * share <= c->sm_count && *std::max_element(lc.begin(), lc.end()) == 0;
     for (int32_t k : order) {
         const JobDev& h = jobs[k]->h;
         const int lg = lc[k], C = 1 << lg;
@@ -1867,11 +1869,14 @@ void group_jobs(const sopb_context* c, sopb_job* const* jobs, int32_t njobs, int
         // noise of 32 beads) as far as they go, in wide lane groups if these
         // still have a warp each
         // One CTA: at most 512 threads where two such CTAs fit an SM's shared
-        // memory, so that their phases overlap (512 replicas of 60 to 600
-        // beads: 5.35 ms per 200 steps, 6.02 with 1024)
+        // memory, so that their phases overlap (512 replicas of 60 to 600 beads:
+        // 5.35 ms per 200 steps, 6.02 with 1024), unless each has an SM to itself
+        // (128 jobs of 200 beads with a tip 1.96 ms with 512, 1.68 with 1024) and
+        // no cluster waits for it (60 jobs of 60 to 600 beads 1.00 ms per 100
+        // steps, 1.27 with 1024)
         int block = h.block;
         bool wide = false;
-        if (block == 1024 && ctas_per_sm(c, 512, smem) > 1) block = 512;
+        if (block == 1024 && !roomy && ctas_per_sm(c, 512, smem) > 1) block = 512;
         if (C > 1) {
             const int nb = local_beads_max(h.n, C), np = (nb + 1) / 2, noise = (nb + 31) / 32, G = std::min(16, 2 * h.lpb);
             wide = h.lpb == 4 && (np + 1) / 2 + noise <= kClusterBlock / 32;
