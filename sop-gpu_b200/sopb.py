@@ -337,14 +337,15 @@ class Context:
         check(lib().sopb_context_sync(self.handle), "sync")
 
     def set_shape_policy(self, lanes_per_bead: int = 4, beads_per_group: float = 1.0, max_block: int = 1024) -> None:
-        """Resident-kernel shape for jobs created from now on (autotuner knob)."""
+        """Resident-kernel shape for jobs created from now on (autotuner knob);
+        a run may give a job fewer threads, or a cluster of CTAs."""
         check(lib().sopb_context_set_shape_policy(self.handle, int(lanes_per_bead), float(beads_per_group),
                                                   int(max_block)), "set_shape_policy")
 
     def set_hi_policy(self, chol_panel_tiles: int = 4, hi_ctas_per_sm: int = 8) -> None:
-        """HI launch policy for jobs created from now on (autotuner knob):
-        exact-HI outer-panel width in 128-column tiles, and the CTAs per SM
-        the O(N^2) HI sums are sliced for."""
+        """Launch policy of exact-HI jobs above 128 beads created from now on
+        (autotuner knob): outer-panel width in 128-column tiles, and the CTAs
+        per SM the D F sums are sliced for."""
         check(lib().sopb_context_set_hi_policy(self.handle, int(chol_panel_tiles), int(hi_ctas_per_sm)),
               "set_hi_policy")
 

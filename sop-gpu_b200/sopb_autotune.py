@@ -6,9 +6,9 @@ will run keeps every job's result independent of what it shares the GPU
 with:
   * the resident kernel's shape (lanes per bead, beads per lane group, CTA
     size cap) for the jobs of up to 2048 beads without HI;
-  * the HI policy of grid-path HI jobs: the exact-HI factorisation's
+  * the HI policy of exact-HI jobs above 128 beads: the factorisation's
     outer-panel width in 128-column tiles and the CTAs per SM that the
-    O(N^2) TEA and D F sums are sliced for.
+    D F sums are sliced for (TEA and smaller exact jobs have none).
 The tuner creates the jobs under each candidate, runs a warm-up, then times
 `repeats` runs of a fixed number of steps on the device and keeps the best
 of them (the runs of one candidate differ by a few per cent; a trial is
@@ -23,7 +23,7 @@ from typing import Iterable, List, Optional, Sequence, Tuple
 import sopb
 
 Policy = Tuple[int, float, int]   # (lanes per bead, beads per lane group, max CTA size)
-HiPolicy = Tuple[int, int]        # (outer-panel tile columns, CTAs per SM of the O(N^2) sums)
+HiPolicy = Tuple[int, int]        # (outer-panel tile columns, CTAs per SM of the D F sums)
 
 DEFAULT_CANDIDATES: List[Policy] = [
     (lpb, bpg, maxb)
@@ -78,11 +78,12 @@ def autotune(ctx: "sopb.Context", specs: Sequence["sopb.JobSpec"], steps: int = 
              candidates: Optional[Iterable[Policy]] = None, log=None, repeats: int = 2,
              hi_steps: int = 20, hi_candidates: Optional[Iterable[HiPolicy]] = None) -> dict:
     """Tunes the resident shape on the mix's resident jobs and the HI policy
-    on its HI jobs (each job kind, exact and TEA, represented by its largest
-    job).  Returns {"policy": best shape, "table": [(policy, s, bead-steps/s)],
-    "hi_policy": best HI policy or None, "hi_table": [...]} and sets both."""
+    on the largest of its exact-HI jobs above 128 beads, the only ones that it
+    concerns.  Returns {"policy": best shape, "table": [(policy, s, bead-steps/s)],
+    "hi_policy": best HI policy or None, "hi_table": [...]} and sets both (a
+    policy without a job in the mix stays as it was)."""
     resident = [s for s in specs if not s.params.hi_on and s.n <= 2048 and not s.params.grid_path]
-    hi = [s for s in specs if s.params.hi_on]
+    hi = [s for s in specs if s.params.hi_on and s.params.hi_exact and s.n > 128]
     out = {"policy": None, "table": [], "hi_policy": None, "hi_table": []}
     if resident:
         beads = sum(s.n for s in resident)
@@ -94,11 +95,7 @@ def autotune(ctx: "sopb.Context", specs: Sequence["sopb.JobSpec"], steps: int = 
         out["policy"] = min(out["table"], key=lambda t: t[1])[0]
         ctx.set_shape_policy(*out["policy"])
     if hi:
-        reps = []
-        for exact in (1, 0):
-            kind = [s for s in hi if bool(s.params.hi_exact) == bool(exact)]
-            if kind:
-                reps.append(max(kind, key=lambda s: s.n))
+        reps = [max(hi, key=lambda s: s.n)]
         beads = sum(s.n for s in reps)
         for pol in (hi_candidates or DEFAULT_HI_CANDIDATES):
             dt = time_hi_policy(ctx, reps, pol, hi_steps, repeats)
