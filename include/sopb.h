@@ -244,21 +244,25 @@ int sopb_context_create(int32_t device, void* stream, sopb_context** out);
 int sopb_context_destroy(sopb_context* ctx);
 /* Shape policy of the resident kernel for jobs created from now on: lanes
  * cooperating on one bead's force sum (a power of two up to 32, default
- * 4), and beads per lane group (default 1; the CTA holds about
- * n / beads_per_group groups, between 64 threads and max_block (default
- * 1024); <= 0 means one bead per group).  The defaults are the fastest
- * shape measured on a batch of 60-600-bead systems.  The autotuner's knob; a job keeps the shape it was
- * created with, so its result is the same alone and in any mix.  No
- * reference counterpart (the reference runs one thread per bead,
- * src/gsop.cuh:13). */
+ * 4), beads per lane group (default 1; a CTA holds about
+ * n / beads_per_group groups; <= 0 means one bead per group), and the most
+ * threads of a CTA (default 1024, at least 64).  A run may give a job fewer
+ * threads (512, so that two jobs share an SM) or, where SMs would idle, a
+ * cluster of up to sixteen CTAs of at most 512 and max_block threads, each
+ * with a share of the beads.  The defaults are the fastest shape measured on
+ * a batch of 60-600-bead systems.  The autotuner's knob; a job keeps the
+ * lanes and the order of sums it was created with, so its result is the same
+ * alone and in any mix.  No reference counterpart (the reference runs one
+ * thread per bead, src/gsop.cuh:13). */
 int sopb_context_set_shape_policy(sopb_context* ctx, int32_t lanes_per_bead, float beads_per_group, int32_t max_block);
 
-/* Launch policy of grid-path HI jobs created from now on: the width of the
- * exact-HI factorisation's outer panels, in 128-column tiles (default 4:
+/* Launch policy of exact-HI jobs above 128 beads created from now on: the
+ * width of the factorisation's outer panels, in 128-column tiles (default 4:
  * each trailing tile is updated once per 512 columns), and the CTAs per SM
- * that the O(N^2) TEA and D F sums are sliced for (default 8).  Both change
- * only the order of floating-point sums; a job keeps the policy it was
- * created with.  The autotuner's knob for HI jobs; no reference counterpart
+ * that the D F sums are sliced for (default 8).  Both change only the order
+ * of floating-point sums; a job keeps the policy it was created with.  TEA
+ * and smaller exact jobs run one split of their own and take no notice.  The
+ * autotuner's knob for HI jobs; no reference counterpart
  * (the reference factorises unblocked, one CTA per trajectory,
  * src/Integrators/bdhitea_kernel.cu:154-190). */
 int sopb_context_set_hi_policy(sopb_context* ctx, int32_t chol_panel_tiles, int32_t hi_ctas_per_sm);
@@ -316,9 +320,10 @@ int sopb_job_step(sopb_job* job, int64_t* step);
 /* Bead count of a job. */
 int sopb_job_size(sopb_job* job, int32_t* n);
 
-/* Launch shape of a job's resident kernel: lanes cooperating on one bead
- * and the CTA size class.  A function of the job alone (not of the batch
- * it runs in); a job's launch class groups it with same-class jobs.  No
+/* Shape of a job in the resident kernel: lanes cooperating on one bead and
+ * the threads of its largest CTA.  Both are functions of the job and of the
+ * shape policy alone, and fix the order of its sums; the CTAs of a run (512
+ * threads, a cluster) depend on what runs with it and change no result.  No
  * reference counterpart (the reference fixes one thread per bead,
  * src/gsop.cuh:13). */
 int sopb_job_shape(sopb_job* job, int32_t* lanes_per_bead, int32_t* block);

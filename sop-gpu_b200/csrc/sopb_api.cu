@@ -84,8 +84,8 @@ inline int64_t grid_cap_nr(const sopb_params& p, int64_t cap_pp, int64_t cap_pl)
 // each: the Verlet rows (mult 2), the near rows (mult 4).
 inline int64_t row_cap(int64_t n, int64_t cap_pl, int mult) { return std::max<int64_t>(1, std::min<int64_t>(n, mult * cap_pl)); }
 
-// Default CTAs per SM that the O(N^2) TEA and D F sums are sliced for (the
-// fastest of 2..32 for TEA and exact HI at 4000 beads on B200).
+// Default CTAs per SM that the D F sums of exact HI above 128 beads are sliced
+// for (the fastest of 2..32 at 4000 beads on B200).
 constexpr int32_t kHiCtasPerSm = 8;
 
 // Shape policy of the resident kernel (see launch_shape).
@@ -93,8 +93,8 @@ struct ShapePolicy {
     int32_t lpb = 4;
     float beads_per_group = 1.0f;
     int32_t max_block = 1024;
-    // grid-path HI jobs: outer-panel width of the exact-HI factorisation (tile
-    // columns) and the CTAs per SM the O(N^2) sums are sliced for
+    // exact HI above 128 beads: outer-panel width of the factorisation (tile
+    // columns) and the CTAs per SM the D F sums are sliced for
     int32_t chol_panel_tiles = kCholPanelTiles;
     int32_t hi_ctas_per_sm = kHiCtasPerSm;
 };
@@ -194,6 +194,8 @@ struct sopb_job {
     int64_t b0 = 0;
     int32_t n = 0;
     JobDev h{};
+    int32_t max_block = 1024;          // the shape policy it was created with
+    float beads_per_group = 1.0f;
     void* dmem = nullptr;
     size_t dbytes = 0;
     // grid path
@@ -292,8 +294,9 @@ float sqrt_threshold(float cut) {
 }
 
 // Lanes per bead and CTA size of a job.  A function of the job and of the
-// context's shape policy only (never of the batch it runs in), so a job's
-// arithmetic is identical alone and in any mix.  The CTA holds about
+// context's shape policy only (never of the batch it runs in), and with it the
+// order of every sum, so a job's arithmetic is identical alone and in any mix,
+// whatever CTAs a run gives it (group_jobs).  The CTA holds about
 // n / beads_per_group lane groups of `lpb` lanes (a power of two, 64..max_block
 // threads): lane groups take beads dynamically, so several beads per group
 // even out the differing list lengths.  sopb_context_set_shape_policy sets
@@ -1699,6 +1702,8 @@ extern "C" int sopb_job_create(sopb_context* c, const sopb_job_desc* d, sopb_job
     CUDA_TRY(cudaEventRecord(j->ev, st));
     j->st = st;
     j->ctx = c;
+    j->max_block = c->policy.max_block;
+    j->beads_per_group = c->policy.beads_per_group;
     j->slot = slot;
     j->b0 = b0;
     j->n = n;
@@ -1854,7 +1859,8 @@ int run_ended(sopb_context* c, cudaStream_t st, RunPlan& plan) {
 // an SM holds, so the class's largest shared-memory request never lowers the
 // residency of its smaller jobs.
 void group_jobs(const sopb_context* c, sopb_job* const* jobs, int32_t njobs, int share, std::vector<LaunchClass>& out) {
-    std::map<int, LaunchClass> cls;   // key: (lanes per bead, wide, cluster; CTA size, CTAs per SM)
+    // key: lanes per bead, wide, cluster; a cluster's largest CTA, or CTA size and CTAs per SM
+    std::map<int64_t, LaunchClass> cls;
     std::vector<int32_t> order(njobs);
     for (int32_t k = 0; k < njobs; ++k) order[k] = k;
     std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) { return jobs[a]->n > jobs[b]->n; });
@@ -1866,8 +1872,8 @@ void group_jobs(const sopb_context* c, sopb_job* const* jobs, int32_t njobs, int
         const int lg = lc[k], C = 1 << lg;
         const size_t smem = resident_layout(h.n, C, h.lcov[lg], h.lnat[lg], h.bsm[lg], h.lcache[lg]).total;
         // a CTA of a cluster: a warp per task of a step (pairs of beads, the
-        // noise of 32 beads) as far as they go, in wide lane groups if these
-        // still have a warp each
+        // noise of 32 beads), or per beads_per_group of them, up to the job's
+        // max_block, in wide lane groups if these still have a warp each
         // One CTA: at most 512 threads where two such CTAs fit an SM's shared
         // memory, so that their phases overlap (512 replicas of 60 to 600 beads:
         // 5.35 ms per 200 steps, 6.02 with 1024), unless each has an SM to itself
@@ -1879,14 +1885,17 @@ void group_jobs(const sopb_context* c, sopb_job* const* jobs, int32_t njobs, int
         if (block == 1024 && !roomy && ctas_per_sm(c, 512, smem) > 1) block = 512;
         if (C > 1) {
             const int nb = local_beads_max(h.n, C), np = (nb + 1) / 2, noise = (nb + 31) / 32, G = std::min(16, 2 * h.lpb);
-            wide = h.lpb == 4 && (np + 1) / 2 + noise <= kClusterBlock / 32;
+            const int most = std::min(kClusterBlock, jobs[k]->max_block) / 32;
+            wide = h.lpb == 4 && (np + 1) / 2 + noise <= most;
             const int per = 32 / (wide ? 2 * G : G);
-            block = 32 * std::min(kClusterBlock / 32, std::max(2, (np + per - 1) / per + noise));
+            const float want = std::ceil((float)((np + per - 1) / per) / std::max(1.0f, jobs[k]->beads_per_group));
+            block = 32 * std::min(most, std::max(2, (int)want + noise));
         }
         // the CTAs of clusters have an SM each, so those of one size share a
         // launch whatever their jobs' sizes (a launch per size would queue on
         // the side streams)
-        LaunchClass& L = cls[((h.lpb * 2 + wide) * 8 + lg) * 4096 + (C > 1 ? 0 : block * 2 + ctas_per_sm(c, block, smem))];
+        LaunchClass& L = cls[(int64_t)((h.lpb * 2 + wide) * 8 + lg) * 65536 +
+                             (C > 1 ? jobs[k]->max_block : block * 32 + ctas_per_sm(c, block, smem))];
         L.block = std::max(L.block, block);
         L.cluster = C;
         L.lpb = h.lpb;
