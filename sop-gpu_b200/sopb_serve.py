@@ -49,25 +49,23 @@ def on_grid_path(spec: "sopb.JobSpec") -> bool:
 def step_cost(spec: "sopb.JobSpec") -> float:
     """Device time of one step of a grid-path job alone, microseconds, on
     B200, which sizes a job's first quantum and orders jobs until its own
-    quanta have been timed: a per-step launch chain, all-pairs O(n^2) sums
-    for HI and, for exact HI, the factorisation amortised over its refresh
-    period -- up to 128 beads one kernel (about 0.023 n^2 us), above it the
-    chain of 3n/128 tile columns (about 3.8 n us) plus the O(n^2) apply --
-    (fitted to 66 us per TEA step and 1.79 ms per exact step with refresh 10
-    at 4000 beads, 71 and 224 us per exact step with refresh 1 at 40 and 90
-    beads, before the cluster kernels, which take 44 us per TEA step and 79 at
-    90 beads), O(n) otherwise."""
+    quanta have been timed.  Without HI the step kernel and the updaters'
+    launches; TEA all pairs; exact HI up to 128 beads one kernel whose factor
+    is a chain of 32-column panels, above that the D F sums and, at every
+    refresh, the chain of 128-column tiles and its trailing updates.  Fitted to
+    8.7 to 104 us from 2500 to 198000 beads without HI, 10 to 44 us from 50 to
+    4000 beads with TEA, 35, 79 and 113 us at 40, 90 and 128 beads with exact HI
+    and a new factor every step, 307 us at 601 beads (refresh 5) and 1.45 ms at
+    4000 (refresh 10)."""
     p, n = spec.params, float(spec.n)
     if not p.hi_on:
-        return 20.0 + 5e-4 * n
-    cost = 40.0 + 2e-6 * n * n
-    if p.hi_exact:
-        refresh = max(1, int(p.hi_refresh))
-        if n <= 128:
-            cost += 25.0 + 0.023 * n * n / refresh
-        else:
-            cost += 8e-6 * n * n + 3.8 * n / refresh
-    return cost
+        return 8.0 + 4.5e-4 * n
+    if not p.hi_exact:
+        return 11.0 + 2e-6 * n * n
+    refresh = max(1, int(p.hi_refresh))
+    if n <= 128:
+        return 12.0 + 0.8 * n / refresh
+    return 25.0 + 1e-5 * n * n + (2.2 * n + 2.3e-4 * n * n) / refresh
 
 
 @dataclasses.dataclass
