@@ -163,7 +163,7 @@ typedef struct sopb_params {
  * Indices are 0-based bead numbers local to the job, as in the .top file.
  */
 typedef struct sopb_job_desc {
-    int32_t n;                         /* beads                               */
+    int32_t n;                         /* beads (2^28 at most without HI)     */
     const float* xyz;                  /* [3n] coordinates, A                 */
     int32_t nbonds;
     const int32_t* bonds;              /* [2*nbonds] (i, j) in .top order     */

@@ -1347,6 +1347,7 @@ extern "C" int sopb_job_create(sopb_context* c, const sopb_job_desc* d, sopb_job
     CUDA_TRY(cudaSetDevice(c->device));
     const int32_t n = d->n;
     const sopb_params& p = d->params;
+    if (!p.hi_on && n > kMaxPairBeads) return SOPB_ERR_UNSUPPORTED;
     reclaim(c, false);
     int64_t b0;
     if (c->free_slots.empty() || !c->beads.alloc(n, &b0)) {
@@ -2254,10 +2255,10 @@ extern "C" int sopb_job_pairlist(sopb_job* j, int32_t possible, int32_t* counts,
                 const auto *re = r + hd.x, *oe = own + ((i & 1) ? hd.z : hd.y);
                 int32_t* to = row.data();
                 for (; own != oe; ++own) {
-                    while (r != re && *r < *own) *to++ = *r++ >> 4;
-                    *to++ = *own >> 4;
+                    while (r != re && *r < *own) *to++ = (int32_t)(*r++ >> 4);
+                    *to++ = (int32_t)(*own >> 4);
                 }
-                while (r != re) *to++ = *r++ >> 4;
+                while (r != re) *to++ = (int32_t)(*r++ >> 4);
                 counts[i] = (int32_t)std::min<int64_t>(to - row.data(), j->h.cap_pl);
                 const int32_t len = std::max(std::min(counts[i], cap), 0);
                 std::copy_n(row.data(), len, rows + (size_t)i * cap);
@@ -2278,7 +2279,7 @@ extern "C" int sopb_job_pairlist(sopb_job* j, int32_t possible, int32_t* counts,
         } else {
             const size_t nr = (size_t)(np + tile - 1) / tile * tile * cap_u;
             std::unique_ptr<int4[]> vh(new int4[np]);
-            std::unique_ptr<int32_t[]> vr(new int32_t[nr]);
+            std::unique_ptr<uint32_t[]> vr(new uint32_t[nr]);
             CUDA_TRY(cudaMemcpyAsync(vh.get(), j->h.gvh, np * sizeof(int4), cudaMemcpyDeviceToHost, c->io));
             CUDA_TRY(cudaMemcpyAsync(vr.get(), j->h.gvr, nr * 4, cudaMemcpyDeviceToHost, c->io));
             SOPB_TRY(io_end(j, false));

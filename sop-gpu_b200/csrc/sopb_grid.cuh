@@ -1027,6 +1027,8 @@ k_g_verlet(JobDev* __restrict__ Jp, GridAux a, int force) {
 // three CTAs per SM: 80 registers without a spill (64 slow the near rebuilds).
 constexpr int kPairWarps = 8;      // warps per CTA
 constexpr int kPairBuf = 512;      // entries of a filtered possible row kept in shared memory
+constexpr int kMaxPairBeads = 1 << 28;   // entries 16 j of 32 bits
+static_assert(16ull * kMaxPairBeads <= 1ull << 32, "row entries");
 
 // The possible partners of a bead within the root of t, increasing, from
 // `o` to `n` of a warp's buffer; the row's entries from k on are still to come.
@@ -1113,9 +1115,9 @@ __device__ __forceinline__ void merge_rows(Filtered& A, Filtered& B, const float
 struct PairRow {
     int32_t* dst;
     int nf, n0, n1;
-    __device__ __forceinline__ void store(int hit, int pos, int entry) const {
+    __device__ __forceinline__ void store(int hit, int pos, uint32_t entry) const {
         pos += hit == 3 ? 0 : (hit == 1 ? nf : nf + n0);
-        if (hit && pos < nf + n0 + n1) dst[pos] = entry;
+        if (hit && pos < nf + n0 + n1) dst[pos] = (int32_t)entry;
     }
 };
 __device__ __forceinline__ PairRow place_row(const JobDev& J, const GridAux& a, int p, int nf, int n0, int n1, int* alloc, int& err) {
@@ -1141,45 +1143,46 @@ __device__ __forceinline__ void row_from_near(const JobDev& J, const GridAux& a,
     const int l = threadIdx.x & 31, rounds = (count + 31) >> 5;
     const unsigned below = (1u << l) - 1u, all = 0xffffffffu;
     int cf = 0, c0 = 0, c1 = 0;
-    auto cand = [&](int u) { return 32 * u + l < count ? nrow[32 * u + l] : 0; };
-    auto take = [&](float4 q, int e, int& at) {
-        const int hit = ((dist2_rn(x0, q) < J.pl_t ? 1 : 0) | (dist2_rn(x1, q) < J.pl_t ? 2 : 0)) & e;
+    auto cand = [&](int u) { return 32 * u + l < count ? (uint32_t)nrow[32 * u + l] : 0u; };
+    auto take = [&](float4 q, uint32_t e, int& at) {
+        const int hit = ((dist2_rn(x0, q) < J.pl_t ? 1 : 0) | (dist2_rn(x1, q) < J.pl_t ? 2 : 0)) & (int)e;
         const unsigned mf = __ballot_sync(all, hit == 3), m0 = __ballot_sync(all, hit == 1), m1 = __ballot_sync(all, hit == 2);
         at = (hit == 3 ? cf : (hit == 1 ? c0 : c1)) + __popc((hit == 3 ? mf : (hit == 1 ? m0 : m1)) & below);
         cf += __popc(mf);
         c0 += __popc(m0);
         c1 += __popc(m1);
-        return (e & ~7) | hit;
+        return (e & ~7u) | (uint32_t)hit;
     };
-    int w[kKeptRounds], place[kKeptRounds];
+    uint32_t w[kKeptRounds];
+    int place[kKeptRounds];
 #pragma unroll
-    for (int u = 0; u < kKeptRounds; ++u) w[u] = u < rounds ? cand(u) : 0;
+    for (int u = 0; u < kKeptRounds; ++u) w[u] = u < rounds ? cand(u) : 0u;
 #pragma unroll
     for (int u = 0; u < kKeptRounds; u += 4)
         if (u < rounds) {
             // four rounds' gathers in flight; an entry 0 hits nothing
             float4 q[4];
 #pragma unroll
-            for (int v = 0; v < 4; ++v) q[v] = J.x[w[u + v] >> 3];
+            for (int v = 0; v < 4; ++v) q[v] = bead_at(reinterpret_cast<const char*>(J.x), 2 * (w[u + v] & ~7u));
 #pragma unroll
             for (int v = 0; v < 4; ++v) w[u + v] = take(q[v], w[u + v], place[u + v]);
         }
     const int kf = cf, k0 = c0, k1 = c1;
     int at;
     for (int u = kKeptRounds; u < rounds; ++u) {
-        const int e = cand(u);
-        take(J.x[e >> 3], e, at);
+        const uint32_t e = cand(u), j = e >> 3;
+        take(J.x[j], e, at);
     }
     const PairRow row = place_row(J, a, p, cf, c0, c1, alloc, err);
 #pragma unroll
     for (int u = 0; u < kKeptRounds; ++u)
-        if (u < rounds) row.store(w[u] & 3, place[u], 2 * (w[u] & ~7));       // 16 j
+        if (u < rounds) row.store(w[u] & 3, place[u], 2 * (w[u] & ~7u));      // 16 j
     cf = kf;
     c0 = k0;
     c1 = k1;
     for (int u = kKeptRounds; u < rounds; ++u) {
-        const int e = cand(u), v = take(J.x[e >> 3], e, at);
-        row.store(v & 3, at, 2 * (v & ~7));
+        const uint32_t e = cand(u), j = e >> 3, v = take(J.x[j], e, at);
+        row.store(v & 3, at, 2 * (v & ~7u));
     }
 }
 
@@ -1192,8 +1195,8 @@ __device__ __forceinline__ void row_from_possible(const JobDev& J, const GridAux
         cf = c0 = c1 = 0;
         merge_rows(A, B, J.x, J.pl_t, [&](int qa, int ba, int qb, int bb, int, unsigned) {
             const unsigned mf = __ballot_sync(all, ba == 3), m0 = __ballot_sync(all, ba == 1), m1 = __ballot_sync(all, bb);
-            store(ba, (ba == 3 ? cf + __popc(mf & below) : c0 + __popc(m0 & below)), 16 * qa);
-            store(bb, c1 + __popc(m1 & below), 16 * qb);
+            store(ba, (ba == 3 ? cf + __popc(mf & below) : c0 + __popc(m0 & below)), 16u * (uint32_t)qa);
+            store(bb, c1 + __popc(m1 & below), 16u * (uint32_t)qb);
             cf += __popc(mf);
             c0 += __popc(m0);
             c1 += __popc(m1);
@@ -1203,9 +1206,9 @@ __device__ __forceinline__ void row_from_possible(const JobDev& J, const GridAux
     refill(A, J.x, J.pl_t);
     refill(B, J.x, J.pl_t);
     const bool whole = A.k >= A.cnt && B.k >= B.cnt;    // both stay as they are for the second pass
-    pass(A, B, [](int, int, int) {});
+    pass(A, B, [](int, int, uint32_t) {});
     const PairRow row = place_row(J, a, p, cf, c0, c1, alloc, err);
-    pass(whole ? A : A0, whole ? B : B0, [&](int hit, int pos, int entry) { row.store(hit, pos, entry); });
+    pass(whole ? A : A0, whole ? B : B0, [&](int hit, int pos, uint32_t entry) { row.store(hit, pos, entry); });
 }
 
 // The near row of pair p; its length, also beyond its capacity.
@@ -1218,9 +1221,9 @@ __device__ __forceinline__ int build_near_row(const JobDev& J, int32_t* nrow, in
         // before a: the lanes below and the second row's own entries below its rank
         const unsigned lower = r < 32 ? (1u << r) - 1u : all;
         const int pa = count + l + __popc(mb & lower);
-        if (ba && pa < cap) nrow[pa] = 8 * qa + ba;
+        if (ba && pa < cap) nrow[pa] = (int32_t)(8u * (uint32_t)qa + (uint32_t)ba);
         const int pb = count + __popc(mb & below) + window_rank(qa, qb);
-        if (bb && pb < cap) nrow[pb] = 8 * qb + 2;
+        if (bb && pb < cap) nrow[pb] = (int32_t)(8u * (uint32_t)qb + 2u);
         count += __popc(ma) + __popc(mb);
     });
     return count;

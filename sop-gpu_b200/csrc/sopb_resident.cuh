@@ -199,7 +199,7 @@ __device__ __forceinline__ RowHead unpack_head(uint2 v) {
 }
 static_assert(kMaxResidentBeads <= 2048, "row counts of 12 bits, byte offsets of 16");
 
-__device__ __forceinline__ float4 bead_at(const char* xb, int off) { return *reinterpret_cast<const float4*>(xb + off); }
+__device__ __forceinline__ float4 bead_at(const char* xb, uint32_t off) { return *reinterpret_cast<const float4*>(xb + off); }
 
 // ---- the forces of a pair of beads ---------------------------------------------
 // The order of a bead's sum is that of V = 4 lpb (at most 32) lanes per pair
@@ -333,9 +333,9 @@ __device__ __forceinline__ void for_partners(const JobDev& J, int i, Visit visit
     } else if (J.gvr) {
         const int4 hd = J.gvh[i >> 1];
         const int32_t* row = J.gvr + (size_t)((i >> 1) / J.tile) * J.tile * J.cap_u + hd.w;
-        for (int k = 0; k < hd.x; ++k) visit(row[k] >> 4);
+        for (int k = 0; k < hd.x; ++k) visit((int)((uint32_t)row[k] >> 4));
         const int32_t* own = row + hd.x + ((i & 1) ? hd.y : 0);
-        for (int k = 0; k < ((i & 1) ? hd.z : hd.y); ++k) visit(own[k] >> 4);
+        for (int k = 0; k < ((i & 1) ? hd.z : hd.y); ++k) visit((int)((uint32_t)own[k] >> 4));
     } else {
         const int32_t* row = J.pl_j + (size_t)i * J.cap_pl;
         for (int k = 0; k < J.pl_cnt[i]; ++k) visit(row[k]);
