@@ -1,5 +1,5 @@
 // sopb_grid.cuh — the grid path: per-step kernels for jobs too large for one
-// CTA (n > ~4096 beads, e.g. a 198k-bead capsid shell) and for jobs with
+// CTA (n > 2048 beads, e.g. a 198k-bead capsid shell) and for jobs with
 // hydrodynamic interactions, whose O(N^2) sums need the whole GPU.
 //
 // One step of a job without hydrodynamics is one kernel (potentials, noise and

@@ -439,7 +439,7 @@ k_chol_apply(JobDev* __restrict__ Jp, GridAux aux) {
 // Then D F (a warp per bead), L g (a warp per row), the fixed beads and the
 // Ermak-McCammon move.  Between refreshes L is read from the tensor.
 // Bound: the serial chain of 3n/32 panels (factor 9000 cycles, solve and send
-// 5000, two cluster barriers).  90 beads, a new factor every step: 80 us a
+// 5000, two cluster barriers).  90 beads, a new factor every step: 79 us a
 // step with the forces, 231 us with a one-CTA factor that kept the matrix in
 // L2 and took two barriers per column.
 constexpr int kSmallPanel = 32;

@@ -931,7 +931,7 @@ __device__ __noinline__ int run_updaters(const JobDev& J, const PartView& V, Ste
 }
 
 // What bounds it, and what it measured (B200, 200 steps).  One CTA per job:
-// issue slots (74 % busy) beside the shared-memory pipe (60 %), and within
+// issue slots (77-78 % busy) beside the shared-memory pipe, and within
 // them the pair terms; 512 replicas of 60 to 600 beads 5.1 ms, 6.95 ms with
 // a row per bead.  Clusters: the dependent chain of a step (about 1200 cycles
 // without any list, the exchange 250 to 900 of them); one job of 200 beads
