@@ -120,6 +120,7 @@ struct RunPlan {
     int share = 1;                // streams that shared the GPU when it was made
     cudaEvent_t done = nullptr;   // the stream's last run ended (a context with runs on several streams)
     uint64_t overlap = 0;         // the context's run count when a run was last seen beside one on this stream
+    bool captured = false;        // a caller's graph launches from the plan's table: it stays as it is
     std::vector<sopb_job*> jobs;
     std::vector<int64_t> steps;
     std::vector<LaunchClass> cls;
@@ -1831,8 +1832,9 @@ bool capturing(cudaStream_t st) {
 // (Queries are allowed beside a stream capture only in the relaxed mode.)
 int streams_sharing(sopb_context* c, cudaStream_t st, RunPlan& plan) {
     ++c->runs;
+    if (capturing(st)) plan.captured = true;
+    if (plan.captured) return plan.share;
     if (c->plans.size() < 2) return 1;
-    if (capturing(st)) return plan.share;   // the plan at hand needs no upload
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
     cudaThreadExchangeStreamCaptureMode(&mode);
     for (auto& kv : c->plans) {
@@ -1973,6 +1975,7 @@ int run_ordered(sopb_context* c, sopb_job* const* jobs, int32_t njobs, const int
         const int share = streams_sharing(c, st, plan);
         const bool same = plan.generation == c->generation && plan.jobs == resident && plan.steps == rsteps && plan.share == share;
         if (!same) {
+            plan.captured = capturing(st);
             plan.share = share;
             plan.generation = c->generation;
             plan.jobs = resident;
